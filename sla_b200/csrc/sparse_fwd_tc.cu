@@ -634,6 +634,24 @@ static EncodeTiledFn get_encode_fn() {
   return fn;
 }
 
+// The driver's encoder needs a current context, which a thread without any runtime call behind it (an autograd worker
+// whose first work is a backward) does not have yet: selecting the device the runtime would use anyway makes it.
+template <typename Encode>
+static int encode_tmap(Encode&& encode) {
+  CUresult r = encode();
+  if (r == CUDA_ERROR_INVALID_CONTEXT || r == CUDA_ERROR_NOT_INITIALIZED) {
+    int dev = 0;
+    SLA_CUDA_OK(cudaGetDevice(&dev));
+    SLA_CUDA_OK(cudaSetDevice(dev));
+    r = encode();
+  }
+  if (r != CUDA_SUCCESS) {
+    set_last_cuda_error(cudaErrorInvalidValue);
+    return SLA_ERR_CUDA;
+  }
+  return SLA_OK;
+}
+
 int make_tmap_3d(CUtensorMap* out, const void* base, int dtype, int D, int L, int BH, int box_rows) {
   return make_tmap_rows(out, base, dtype, D, L, BH, size_t(L) * D * 2, box_rows);
 }
@@ -647,14 +665,11 @@ int make_tmap_rows(CUtensorMap* out, const void* base, int dtype, int D, int L, 
   cuuint64_t strides[2] = {static_cast<cuuint64_t>(D) * 2, static_cast<cuuint64_t>(head_stride_bytes)};
   cuuint32_t box[3] = {64, static_cast<cuuint32_t>(box_rows), 1};
   cuuint32_t estr[3] = {1, 1, 1};
-  CUresult r = fn(out, dtype == SLA_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3,
-                  const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) {
-    set_last_cuda_error(cudaErrorInvalidValue);
-    return SLA_ERR_CUDA;
-  }
-  return SLA_OK;
+  return encode_tmap([&]() {
+    return fn(out, dtype == SLA_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3,
+              const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  });
 }
 
 int make_tmap_3d_u8(CUtensorMap* out, const void* base, int row_bytes, int L, int BH, int box_rows) {
@@ -664,14 +679,11 @@ int make_tmap_3d_u8(CUtensorMap* out, const void* base, int row_bytes, int L, in
   cuuint64_t strides[2] = {static_cast<cuuint64_t>(row_bytes), static_cast<cuuint64_t>(L) * row_bytes};
   cuuint32_t box[3] = {static_cast<cuuint32_t>(row_bytes), static_cast<cuuint32_t>(box_rows), 1};
   cuuint32_t estr[3] = {1, 1, 1};
-  CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void*>(base), dims, strides, box, estr,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) {
-    set_last_cuda_error(cudaErrorInvalidValue);
-    return SLA_ERR_CUDA;
-  }
-  return SLA_OK;
+  return encode_tmap([&]() {
+    return fn(out, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void*>(base), dims, strides, box, estr,
+              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  });
 }
 
 constexpr int kFwdStaticSmem = 2 * 1024;   // statically allocated shared memory of the kernel (barriers, z, bias, 1/den)
