@@ -11,12 +11,16 @@
 //
 // Roles (576 threads, one CTA per SM):
 //   warps 0-15  four compute groups of 128 threads (thread = tile row = TMEM lane). Group g works on
-//               entries j = g & 1 (mod 2) in TMEM buffer g & 1 and on the 32 score columns
+//               entries j = g & 1 (mod 2) and on the 32 score columns
 //               [32 (g >> 1), +32): it reads T1, T2, forms P and dS (the backward has no cross-entry or
 //               cross-column state) and writes them back as 16-bit A operands over its own columns.
 //   warp 16     TMA producer (stationary tiles once, then a ring of streamed tiles + row stats)
 //   warp 17     MMA issuer.
-// TMEM: acc1 [0,D) (dK), acc2 [D,2D) (dV), then per buffer T1 (64 cols), T2 (64 cols).
+// TMEM: acc1 [0,D) (dK), acc2 [D,2D) (dV), then per buffer T1 (64 cols), T2 (64 cols); entry j uses buffer j mod NB.
+// The 512 columns hold two buffers at head dim 128 and three at 64. With as many buffers as compute pairs a pair waits
+// for the accumulation GEMMs of its own entry and the scores of its next one; a third buffer has those scores ready
+// before the pair is done with its entry, which matters at head dim 64, where the GEMMs are short and the chain
+// compute -> accumulate -> scores is what a pair waits on.
 // Row statistics (lse, delta) come from a padded (B*H, Lpad, 2) fp32 array written by the dQ kernel, which runs
 // first (delta = rowsum(o_s * dO), kernel.py:102-105; padding rows hold lse = +inf).
 // All waits are bounded; see tc_common.cuh.
@@ -78,9 +82,10 @@ sparse_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_co
   constexpr uint32_t IDESC_ACC = idesc_f16(FMT, 128, D, 0, 1);
   constexpr uint32_t TMEM_COLS = 512;
   constexpr int COL_ACC1 = 0, COL_ACC2 = D, COL_T = 2 * D;
+  constexpr int NB = (512 - 2 * D) / 128;                    // score buffers
 
   extern __shared__ uint8_t smem_raw[];
-  __shared__ __align__(8) uint64_t bars[2 * NS + 10];
+  __shared__ __align__(8) uint64_t bars[2 * NS + 2 * NB + 6];
   __shared__ float s_dz[D];                        // fused linear backward: gradient of z
   __shared__ float s_e[3][4][128];                 // row-wide maxima / sums handed between the four compute groups
   __shared__ uint32_t s_tmem_base;
@@ -103,10 +108,10 @@ sparse_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_co
 
   const uint32_t bar0 = smem_u32(&bars[0]);
   auto BAR = [&](int i) { return bar0 + 8u * i; };
-  // 0 x_full | 1..NS y_full | NS+1..2NS y_empty | then t_full[2], c_full[2], acc_done
-  constexpr int B_X = 0, B_YF = 1, B_YE = 1 + NS, B_T = 1 + 2 * NS, B_C = 3 + 2 * NS, B_ACC = 5 + 2 * NS;
+  // 0 x_full | 1..NS y_full | NS+1..2NS y_empty | then t_full[NB], c_full[NB], acc_done
+  constexpr int B_X = 0, B_YF = 1, B_YE = 1 + NS, B_T = 1 + 2 * NS, B_C = B_T + NB, B_ACC = B_C + NB;
   // fused linear dk, dv: dH landed in stage 0 | phi(k) written over the K tile | the two GEMMs done
-  constexpr int B_DH = 7 + 2 * NS, B_PHIK = 8 + 2 * NS, B_LIN = 9 + 2 * NS;
+  constexpr int B_DH = B_ACC + 1, B_PHIK = B_ACC + 2, B_LIN = B_ACC + 3;
   const bool lin = p.lin_feature >= 0;
 
   if (warp == 16 && lane == 0) {
@@ -117,7 +122,7 @@ sparse_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_co
       mbar_init(BAR(B_YF + s), 1);
       mbar_init(BAR(B_YE + s), 1);
     }
-    for (int b = 0; b < 2; ++b) {
+    for (int b = 0; b < NB; ++b) {
       mbar_init(BAR(B_T + b), 1);
       mbar_init(BAR(B_C + b), 8);      // one arrival per warp of the buffer's two compute groups
     }
@@ -224,7 +229,7 @@ sparse_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_co
       long long* trm = lane == 0 ? tr : nullptr;
       const uint32_t x1_lo = desc_lo(sX1, 16), x2_lo = desc_lo(sX2, 16);
       auto issue_t = [&](int j) {
-        const int s = j % NS, b = j & 1;
+        const int s = j % NS, b = j % NB;
         const uint32_t y1_lo = desc_lo(sY0 + s * 2 * Y_BYTES, 16), y2_lo = desc_lo(sY0 + s * 2 * Y_BYTES + Y_BYTES, 16);
         const uint32_t t1 = tmem + COL_T + b * 128, t2 = t1 + 64;
         if (elect_one()) {
@@ -243,16 +248,16 @@ sparse_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_co
         __syncwarp();
       };
       bool ok = warp_all(mbar_wait(BAR(B_X), 0, kBErrX, p.err));
-      for (int j = 0; ok && j < 2 && j < n_ent; ++j) {
+      for (int j = 0; ok && j < NB && j < n_ent; ++j) {
         ok = warp_all(mbar_wait(BAR(B_YF + j % NS), (j / NS) & 1, kBErrYFull, p.err));
         if (!ok) break;
         tc_fence_after();
         issue_t(j);
       }
       for (int j = 0; ok && j < n_ent; ++j) {
-        const int s = j % NS, b = j & 1;
+        const int s = j % NS, b = j % NB;
         trace_ev(trm, 1, j, 0);
-        ok = warp_all(mbar_wait(BAR(B_C + b), (j >> 1) & 1, kBErrCFull, p.err));
+        ok = warp_all(mbar_wait(BAR(B_C + b), (j / NB) & 1, kBErrCFull, p.err));
         if (!ok) break;
         trace_ev(trm, 1, j, 1);
         tc_fence_after();
@@ -273,11 +278,11 @@ sparse_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_co
         }
         __syncwarp();
         trace_ev(trm, 1, j, 2);
-        if (j + 2 < n_ent) {
-          ok = warp_all(mbar_wait(BAR(B_YF + (j + 2) % NS), ((j + 2) / NS) & 1, kBErrYFull, p.err));
+        if (j + NB < n_ent) {
+          ok = warp_all(mbar_wait(BAR(B_YF + (j + NB) % NS), ((j + NB) / NS) & 1, kBErrYFull, p.err));
           if (!ok) break;
           tc_fence_after();
-          issue_t(j + 2);
+          issue_t(j + NB);
         }
         trace_ev(trm, 1, j, 3);
       }
@@ -317,7 +322,7 @@ sparse_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_co
   } else {
     // ------------------------------ compute groups ------------------------------
     const int wg = warp >> 2;                               // 0..3
-    const int buf = wg & 1, ch = wg >> 1;                   // TMEM buffer, column half
+    const int ch = wg >> 1;                                 // column half
     const int row = tid & 127;                              // tile row == TMEM lane
     const uint32_t lane_addr = static_cast<uint32_t>((warp & 3) * 32) << 16;
     const int half = row >> 6;
@@ -325,10 +330,14 @@ sparse_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_co
     const int grow = tile * 128 + row;                      // global key row
     const bool key_ok = grow < L;                           // keys past the end give P = 0 (kernel.py:216)
     bool ok = !*abortp;
-    for (int j = buf; ok && j < n_ent; j += 2) {
+    // A pair meets a buffer again after lcm(2, NB) entries, the other pair having used it in between; the scores are
+    // computed in order, so when a pair waits for entry j's it knows that those of entry j - NB are there, and the
+    // parity of the phase is enough.
+    for (int j = wg & 1; ok && j < n_ent; j += 2) {
+      const int buf = NB == 2 ? (wg & 1) : j % NB;
       long long* trc = ((warp & 3) == 0 && lane == 0) ? tr : nullptr;
       trace_ev(trc, 2 + ch, j, 0);
-      if (!mbar_wait(BAR(B_T + buf), (j >> 1) & 1, kBErrTFull, p.err)) { ok = false; break; }
+      if (!mbar_wait(BAR(B_T + buf), (j / NB) & 1, kBErrTFull, p.err)) { ok = false; break; }
       if (*abortp) { ok = false; break; }
       trace_ev(trc, 2 + ch, j, 1);
       if (!mbar_wait(BAR(B_YF + j % NS), (j / NS) & 1, kBErrYFull, p.err)) { ok = false; break; }  // row stats landed
