@@ -267,11 +267,18 @@ int sla_ipc_close(void* ptr) {
   return SLA_OK;
 }
 
+// Order of the dK/dV kernel's key tiles in the sparse backward's workspace; `order` stays NULL where it does not pay.
+static TileOrder bwd_tile_order(const sla_shape* s, const int32_t* col_offsets, unsigned char* sparse_ws) {
+  return make_tile_order(col_offsets, reinterpret_cast<int32_t*>(sparse_ws + ws_sparse_bwd(s).order),
+                         ceil_div(s->L, s->BLKK), ceil_div(s->L, s->BLKQ), s->D, s->B * s->H);
+}
+
+// `ordered`: the linear branch's reductions have made the tile order already.
 static int sparse_bwd_impl(const sla_shape* s, const void* q, const void* k, const void* v, const void* o_s,
                            const float* lse, const void* do_s, const int32_t* lut, const int32_t* col_offsets,
                            const int32_t* col_index, void* dq, void* dk, void* dv, unsigned char* ws,
                            int accumulate_legacy, cudaStream_t st, const void* lin_dh = nullptr,
-                           const float* lin_dz = nullptr) {
+                           const float* lin_dz = nullptr, bool ordered = false) {
   WsSparseBwd w = ws_sparse_bwd(s);
   BwdParams p;
   p.q = q; p.k = k; p.v = v; p.o_s = o_s; p.d_o = do_s; p.lse = lse;
@@ -281,6 +288,12 @@ static int sparse_bwd_impl(const sla_shape* s, const void* q, const void* k, con
   p.scale = softmax_scale(s); p.scale_log2 = p.scale * kLog2e; p.accumulate = accumulate_legacy;
   p.lin_dh = lin_dh; p.lin_dz = lin_dz;
   if (!(s->flags & SLA_FLAG_LEGACY_MMA)) {
+    const TileOrder order = bwd_tile_order(s, col_offsets, ws);
+    if (order.order && !ordered && sparse_bwd_tc_fits(s)) {
+      int rc = run_tile_order(order, st);
+      if (rc != SLA_OK) return rc;
+    }
+    p.order = order;
     int rc = run_sparse_bwd_tc(s, p, ws + w.stats, st);
     if (rc != SLA_ERR_BAD_SHAPE) return rc;   // lists too long for the tcgen05 kernel's shared memory
   }
@@ -328,6 +341,7 @@ static int bwd_unselected(const sla_shape* s, const void* q, const void* k, cons
   lp.dw_part = reinterpret_cast<float*>(base + wb.dw_part);
   lp.dw = dw; lp.dbias = dbias; lp.L = s->L; lp.nch = wb.nch; lp.rows = wb.rows;
   lp.g_stride = 2 * s->D * s->D + 2 * s->D; lp.has_g2 = 1;
+  lp.order = bwd_tile_order(s, col_offsets, sparse_ws);
   if ((rc = run_linear_bwd_reductions(s, lp, st)) != SLA_OK) return rc;
   // the product without softmax over the selected blocks, on (phi(q), phi(k), v) with dO = -dN, delta = dden:
   // dq += dS phi(k) (still a gradient of phi(q)); dk = phi'(k)(v dH^T + dz + dS^T phi(q)); dv = phi(k) dH + P^T dO
@@ -338,10 +352,12 @@ static int bwd_unselected(const sla_shape* s, const void* q, const void* k, cons
   bp.L = s->L; bp.mb = ceil_div(s->L, s->BLKQ); bp.nb = nb; bp.topk = s->topk;
   bp.scale = 1.0f; bp.scale_log2 = 1.0f; bp.accumulate = 1;
   bp.lin_dh = lp.dh; bp.lin_dz = lp.dz; bp.plain = 1;
+  bp.order = lp.order;
   if ((rc = run_sparse_bwd_tc(s, bp, ub + wu.stats, st)) != SLA_OK) return rc;
   if ((rc = run_feature_map_bwd(s, ub + wu.phiq, dq, st)) != SLA_OK) return rc;   // dq = phi'(q) dphi_q
   // the softmax branch adds its dq, dk, dv
-  return sparse_bwd_impl(s, q, k, v, o_s, lse, d_o, lut, col_offsets, col_index, dq, dk, dv, sparse_ws, 1, st);
+  return sparse_bwd_impl(s, q, k, v, o_s, lse, d_o, lut, col_offsets, col_index, dq, dk, dv, sparse_ws, 1, st,
+                         nullptr, nullptr, true);
 }
 
 int sla_sparse_bwd(const sla_shape* s, const void* q, const void* k, const void* v, const void* o_s,
@@ -401,10 +417,11 @@ int sla_bwd(const sla_shape* s, const void* q, const void* k, const void* v, con
   lp.accumulate = 0;
   lp.skip_kv = fuse_kv ? 1 : 0;
   lp.tc_pass_a = legacy ? 0 : 1;
+  if (fuse_kv) lp.order = bwd_tile_order(s, col_offsets, sparse_ws);
   rc = run_linear_bwd(s, lp, st);
   if (rc != SLA_OK || linear_only) return rc;
   return sparse_bwd_impl(s, q, k, v, o_s, lse, d_o, lut, col_offsets, col_index, dq, dk, dv, sparse_ws, 1, st,
-                         fuse_kv ? lp.dh : nullptr, fuse_kv ? lp.dz : nullptr);
+                         fuse_kv ? lp.dh : nullptr, fuse_kv ? lp.dz : nullptr, fuse_kv);
 }
 
 }  // extern "C"

@@ -4,6 +4,7 @@
 #include <stdint.h>
 
 #include "../../include/sla_b200.h"
+#include "tile_order.cuh"
 
 namespace sla {
 
@@ -45,6 +46,7 @@ struct BwdParams {
   // with `delta` given by the caller in the row statistics (no pre-pass), no softmax scale. With lin_dh set, q and k
   // are feature maps already and dk = phi'(k) (v dH^T + dz + dK), dv = phi(k) dH + dV.
   int plain = 0;
+  TileOrder order;        // tcgen05 path only: order of the dK/dV kernel's last key tiles, order.order made beforehand
 };
 
 struct LinBwdParams {
@@ -67,6 +69,7 @@ struct LinBwdParams {
   // g_stride floats {G, dz, db, G2}, and the head's dW is G H - G2
   int g_stride = 0;       // 0: the default record D*D + 2*D
   int has_g2 = 0;
+  TileOrder order;        // made by the first reduction kernel on the side when order.order is set
 };
 
 // Row pass of the backward of the "unselected" linear scope.
@@ -95,6 +98,7 @@ int run_state_proj(const sla_shape* s, void* lin_state, const void* wbits, cudaS
 int read_tc_error(int* out, bool clear);
 void set_trace_buffer(long long* p);
 long long* trace_buffer();
+int run_tile_order(const TileOrder& o, cudaStream_t st);
 int run_sparse_bwd_tc(const sla_shape* s, const BwdParams& p, void* stats, cudaStream_t st);
 bool sparse_bwd_tc_fits(const sla_shape* s);
 bool sparse_bwd_dq_pair_fits(const sla_shape* s);

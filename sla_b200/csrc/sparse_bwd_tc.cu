@@ -24,6 +24,7 @@
 // Row statistics (lse, delta) come from a padded (B*H, Lpad, 2) fp32 array written by the dQ kernel, which runs
 // first (delta = rowsum(o_s * dO), kernel.py:102-105; padding rows hold lse = +inf).
 // All waits are bounded; see tc_common.cuh.
+#include <limits.h>
 #include <type_traits>
 
 #include "common.cuh"
@@ -45,6 +46,8 @@ struct TcBwdParams {
   // the linear branch's dk, dv computed in the epilogue (feature < 0: not fused)
   int lin_feature;           // sla_feature or -1
   const float* dz;           // [BH][D] fp32 gradient of z = sum phi(k)
+  const int32_t* order;      // CTAs from order_from on: CTA - order_from -> head * tiles + tile (tile_order.cuh)
+  int order_from;
 };
 
 __device__ __forceinline__ float ex2b(float x) {
@@ -93,9 +96,20 @@ sparse_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_co
   __shared__ int s_abort;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int tile = blockIdx.x, bh = blockIdx.y;
   const int L = p.L;
   pdl_entry();
+  // {tile, head} this CTA works on, looked up again at every use: kept in registers or handed on through shared memory
+  // they make the compute groups spill.
+  struct Unit {
+    const TcBwdParams& p;
+    __device__ __forceinline__ int operator[](int w) const {
+      const int lin_id = blockIdx.y * gridDim.x + blockIdx.x;
+      const int id = lin_id >= p.order_from ? *reinterpret_cast<const volatile int*>(p.order + (lin_id - p.order_from)) : lin_id;
+      const int head = id / static_cast<int>(gridDim.x);
+      return w ? head : id - head * static_cast<int>(gridDim.x);
+    }
+  };
+  const Unit unit{p};
 
   const uint32_t raw_a = smem_u32(smem_raw);
   const uint32_t base_a = (raw_a + 1023u) & ~1023u;
@@ -114,33 +128,34 @@ sparse_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_co
   constexpr int B_DH = B_ACC + 1, B_PHIK = B_ACC + 2, B_LIN = B_ACC + 3;
   const bool lin = p.lin_feature >= 0;
 
-  if (warp == 16 && lane == 0) {
-    // the producer lane sets the barriers up itself and requests the stationary tiles before it merges the lists
-    s_abort = *reinterpret_cast<volatile int*>(p.err) != 0;
-    mbar_init(BAR(B_X), 1);
-    for (int s = 0; s < NS; ++s) {
-      mbar_init(BAR(B_YF + s), 1);
-      mbar_init(BAR(B_YE + s), 1);
-    }
-    for (int b = 0; b < NB; ++b) {
-      mbar_init(BAR(B_T + b), 1);
-      mbar_init(BAR(B_C + b), 8);      // one arrival per warp of the buffer's two compute groups
-    }
-    mbar_init(BAR(B_ACC), 1);
-    mbar_init(BAR(B_DH), 1);
-    mbar_init(BAR(B_PHIK), 16);
-    mbar_init(BAR(B_LIN), 1);
-    fence_barrier_init();
-    fence_proxy_async_smem();
-    if (!s_abort) {
-      mbar_expect_tx(BAR(B_X), 2 * X_BYTES);
-      for (int c = 0; c < SLABS; ++c) {
-        tma_load_3d(sX1 + c * X_SLAB, &tmX1, BAR(B_X), c * 64, tile * 128, bh);
-        tma_load_3d(sX2 + c * X_SLAB, &tmX2, BAR(B_X), c * 64, tile * 128, bh);
+  if (warp == 16) {
+    const int tile = unit[0], bh = unit[1];
+    if (lane == 0) {
+      // the producer lane sets the barriers up itself and requests the stationary tiles before it merges the lists
+      s_abort = *reinterpret_cast<volatile int*>(p.err) != 0;
+      mbar_init(BAR(B_X), 1);
+      for (int s = 0; s < NS; ++s) {
+        mbar_init(BAR(B_YF + s), 1);
+        mbar_init(BAR(B_YE + s), 1);
+      }
+      for (int b = 0; b < NB; ++b) {
+        mbar_init(BAR(B_T + b), 1);
+        mbar_init(BAR(B_C + b), 8);      // one arrival per warp of the buffer's two compute groups
+      }
+      mbar_init(BAR(B_ACC), 1);
+      mbar_init(BAR(B_DH), 1);
+      mbar_init(BAR(B_PHIK), 16);
+      mbar_init(BAR(B_LIN), 1);
+      fence_barrier_init();
+      fence_proxy_async_smem();
+      if (!s_abort) {
+        mbar_expect_tx(BAR(B_X), 2 * X_BYTES);
+        for (int c = 0; c < SLABS; ++c) {
+          tma_load_3d(sX1 + c * X_SLAB, &tmX1, BAR(B_X), c * 64, tile * 128, bh);
+          tma_load_3d(sX2 + c * X_SLAB, &tmX2, BAR(B_X), c * 64, tile * 128, bh);
+        }
       }
     }
-  }
-  if (warp == 16) {
     if (lane == 0) {
       prefetch_tmap(&tmX1); prefetch_tmap(&tmX2); prefetch_tmap(&tmY1); prefetch_tmap(&tmY2);
       prefetch_tmap(&tmO1); prefetch_tmap(&tmO2);
@@ -169,14 +184,14 @@ sparse_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_co
     tmem_alloc(smem_u32(&s_tmem_base), TMEM_COLS);
     tmem_relinquish();
   }
-  if (lin && tid < D) s_dz[tid] = p.dz[static_cast<size_t>(bh) * D + tid];
+  if (lin && tid < D) s_dz[tid] = p.dz[static_cast<size_t>(unit[1]) * D + tid];
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = s_tmem_base;
   const int n_ent = s_n_entries * SL;            // streamed 64-row tiles
   volatile int* abortp = &s_abort;
-  long long* tr = (tile == 0 && bh == 0) ? p.trace : nullptr;
+  long long* tr = (unit[0] == 0 && unit[1] == 0) ? p.trace : nullptr;
 
   // global row of the streamed tile j
   auto y_row0 = [&](int j) {
@@ -187,6 +202,7 @@ sparse_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_co
   if (warp == 16) {
     // ------------------------------ TMA producer ------------------------------
     if (lane == 0 && !*abortp) {
+      const int bh = unit[1];
       int issued = 0;
       for (int j = 0; j < n_ent; ++j) {
         const int s = j % NS, use = j / NS;
@@ -327,8 +343,7 @@ sparse_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_co
     const uint32_t lane_addr = static_cast<uint32_t>((warp & 3) * 32) << 16;
     const int half = row >> 6;
     const float sc = p.scale_log2;
-    const int grow = tile * 128 + row;                      // global key row
-    const bool key_ok = grow < L;                           // keys past the end give P = 0 (kernel.py:216)
+    const bool key_ok = unit[0] * 128 + row < L;                           // keys past the end give P = 0 (kernel.py:216)
     bool ok = !*abortp;
     // A pair meets a buffer again after lcm(2, NB) entries, the other pair having used it in between; the scores are
     // computed in order, so when a pair waits for entry j's it knows that those of entry j - NB are there, and the
@@ -439,7 +454,7 @@ sparse_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_co
             else x[c] = x[c] > 0.f ? x[c] + 1.f : __expf(x[c]);      // elu(x) + 1
           }
         }
-        const bool key_live = grow < L;                        // rows past the end: K was zero-filled, phi must be 0
+        const bool key_live = unit[0] * 128 + row < L;                        // rows past the end: K was zero-filled, phi must be 0
         uint32_t phi[CW / 2];                                  // phi(k) rounded to T (core.py:91)
 #pragma unroll
         for (int c = 0; c < CW; c += 2) phi[c >> 1] = key_live ? Elem<T>::pack2(x[c], x[c + 1]) : 0u;
@@ -514,8 +529,8 @@ sparse_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_co
         asm volatile("bar.sync 1, 512;\n" ::: "memory");
         if (tid == 0 && !*abortp) {
           for (int c = 0; c < SLABS; ++c) {
-            tma_store_3d(&tmO1, sX1 + c * X_SLAB, c * 64, tile * 128, bh);
-            tma_store_3d(&tmO2, sX2 + c * X_SLAB, c * 64, tile * 128, bh);
+            tma_store_3d(&tmO1, sX1 + c * X_SLAB, c * 64, unit[0] * 128, unit[1]);
+            tma_store_3d(&tmO2, sX2 + c * X_SLAB, c * 64, unit[0] * 128, unit[1]);
           }
           tma_store_commit();
           tma_store_wait_read();
@@ -556,11 +571,11 @@ sparse_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_co
       asm volatile("bar.sync 1, 512;\n" ::: "memory");
       if (tid == 0) {
         if (p.accumulate) {   // read-modify-write done by the copy engine in L2: no load stalls this CTA
-          for (int c = 0; c < SLABS; ++c) tma_reduce_add_3d(&tmO1, sX1 + c * X_SLAB, c * 64, tile * 128, bh);
-          for (int c = 0; c < SLABS; ++c) tma_reduce_add_3d(&tmO2, sX2 + c * X_SLAB, c * 64, tile * 128, bh);
+          for (int c = 0; c < SLABS; ++c) tma_reduce_add_3d(&tmO1, sX1 + c * X_SLAB, c * 64, unit[0] * 128, unit[1]);
+          for (int c = 0; c < SLABS; ++c) tma_reduce_add_3d(&tmO2, sX2 + c * X_SLAB, c * 64, unit[0] * 128, unit[1]);
         } else {
-          for (int c = 0; c < SLABS; ++c) tma_store_3d(&tmO1, sX1 + c * X_SLAB, c * 64, tile * 128, bh);
-          for (int c = 0; c < SLABS; ++c) tma_store_3d(&tmO2, sX2 + c * X_SLAB, c * 64, tile * 128, bh);
+          for (int c = 0; c < SLABS; ++c) tma_store_3d(&tmO1, sX1 + c * X_SLAB, c * 64, unit[0] * 128, unit[1]);
+          for (int c = 0; c < SLABS; ++c) tma_store_3d(&tmO2, sX2 + c * X_SLAB, c * 64, unit[0] * 128, unit[1]);
         }
         tma_store_commit();
         tma_store_wait_read();
@@ -584,6 +599,16 @@ sparse_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_co
 static long long* g_trace_buffer = nullptr;
 void set_trace_buffer(long long* p) { g_trace_buffer = p; }
 long long* trace_buffer() { return g_trace_buffer; }
+
+__global__ void __launch_bounds__(kOrderThreads) tile_order_kernel(TileOrder o) {
+  pdl_entry();
+  order_tiles(o);
+}
+int run_tile_order(const TileOrder& o, cudaStream_t st) {
+  SLA_CUDA_OK(launch_pdl(tile_order_kernel, dim3(1), dim3(kOrderThreads), 0, st, o));
+  SLA_LAUNCH_OK();
+  return SLA_OK;
+}
 
 static int bwd_tc_smem_bytes(int D, int max_entries) {
   const int NS = D == 128 ? 4 : 6;
@@ -616,6 +641,8 @@ static int launch_dkdv(const sla_shape* s, const BwdParams& bp, const float2* st
   p.scale = bp.scale; p.scale_log2 = bp.scale_log2; p.accumulate = bp.accumulate;
   p.lin_feature = lin ? s->feature_map : -1;
   p.dz = bp.lin_dz;
+  p.order = bp.order.order;
+  p.order_from = bp.order.order ? bp.order.h0 * bp.order.ntiles : INT_MAX;
   p.max_entries = 2 * bp.mb;            // a KV block may have been selected by every query block
   const int smem = bwd_tc_smem_bytes(D, p.max_entries);
   if (smem + kBwdStaticSmem > 227 * 1024) return SLA_ERR_BAD_SHAPE;

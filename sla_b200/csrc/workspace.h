@@ -114,10 +114,11 @@ inline WsBwd ws_bwd(const sla_shape* s) {
   return w;
 }
 
-// ---- sparse backward: padded row statistics {lse, delta} and the plain delta array ----
+// ---- sparse backward: padded row statistics {lse, delta}, the plain delta array, the tile order ----
 struct WsSparseBwd {
   size_t stats;   // float2 [BH][Lpad], Lpad = ceil(L/128)*128
   size_t delta;   // fp32 [BH][L]
+  size_t order;   // int32, at most [BH][ceil(N_BLOCKS / 2)]: order of the last key tiles
   size_t total;
 };
 inline WsSparseBwd ws_sparse_bwd(const sla_shape* s) {
@@ -127,6 +128,7 @@ inline WsSparseBwd ws_sparse_bwd(const sla_shape* s) {
   size_t o = 0;
   w.stats = o; o += ws_round(bh * lpad * 8);
   w.delta = o; o += ws_round(bh * size_t(s->L) * 4);
+  w.order = o; o += ws_round(bh * ws_ceil_div(ws_ceil_div(s->L, s->BLKK), 2) * 4);
   w.total = o;
   return w;
 }

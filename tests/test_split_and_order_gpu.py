@@ -18,6 +18,26 @@ def _randn(shape, seed, dtype=torch.bfloat16):
     return torch.randn(shape, generator=g, device="cuda").to(dtype)
 
 
+@pytest.mark.parametrize("L,D,BLKQ,heads", [(1000, 64, 64, 24), (2500, 128, 128, 9), (19000, 64, 128, 3)])
+def test_tile_order_leaves_the_gradients_alone(L, D, BLKQ, heads):
+    """All heads in one call take the ordered tiles (more than one per SM), a head by itself the sequence order."""
+    q, k, v, do = (_randn((1, heads, L, D), 10 + i) for i in range(4))
+    k[:, :, : L // 3] *= 3                                # popular and unpopular blocks
+
+    def grads(h0, h1):
+        qs, ks, vs = (t[:, h0:h1].contiguous().requires_grad_(True) for t in (q, k, v))
+        smap, lut, topk = sla_b200.get_block_map(qs.detach(), ks.detach(), 0.2, BLKQ, 64)
+        sla_b200._attention.apply(qs, ks, vs, smap, lut, topk, BLKQ, 64).backward(do[:, h0:h1].contiguous())
+        return qs.grad, ks.grad, vs.grad
+
+    tiles = (((L + 63) // 64) + 1) // 2
+    assert tiles * heads > 148 and (tiles <= 148 or D == 64)
+    whole = grads(0, heads)
+    for h in range(heads):
+        for a, b in zip(whole, grads(h, h + 1)):
+            assert torch.equal(a[:, h], b[:, 0])
+
+
 def test_first_call_of_a_thread_may_be_a_backward():
     """A new process, whose autograd thread has made no CUDA call when the backward encodes its tensor maps."""
     code = """
