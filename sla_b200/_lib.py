@@ -14,13 +14,13 @@ LIB_PATH = os.path.join(_HERE, "libsla_b200.so")
 SLA_BF16, SLA_FP16, SLA_FP32 = 0, 1, 2
 PHI = {"softmax": 0, "relu": 1, "elu": 2}
 OP_BLOCK_MAP, OP_FWD, OP_BWD, OP_LINEAR_STATE, OP_SAGE_FWD, OP_SPARSE_BWD = 0, 1, 2, 3, 4, 5
-FLAG_SPARSE_ONLY, FLAG_LEGACY_MMA, FLAG_LINEAR_UNSELECTED, FLAG_STATE_READY, FLAG_LINEAR_ONLY = 1, 2, 4, 8, 16
+FLAG_SPARSE_ONLY, FLAG_LEGACY_MMA, FLAG_LINEAR_UNSELECTED, FLAG_STATE_READY, FLAG_LINEAR_ONLY, FLAG_FWD_SAVED = 1, 2, 4, 8, 16, 32
 
 # every symbol include/sla_b200.h declares
 EXPORTS = (
     "sla_version", "sla_status_string", "sla_last_cuda_error", "sla_launch_count", "sla_poll_device_error", "sla_debug_set_trace", "sla_debug_set_wait_limit_ns", "sla_debug_drop_first_k_tile", "sla_topk_count", "sla_workspace_bytes", "sla_kernel_path",
     "sla_block_map", "sla_column_lists", "sla_index_convert", "sla_pooled_sums_bytes", "sla_qk_norm_rope_pool",
-    "sla_block_map_pooled", "sla_sparse_fwd", "sla_sparse_bwd", "sla_linear_state", "sla_linear_state_static", "sla_fwd", "sla_fwd_gather", "sla_enable_peer_access", "sla_ipc_export", "sla_ipc_open", "sla_ipc_close", "sla_fwd_prepare", "sla_bwd",
+    "sla_block_map_pooled", "sla_sparse_fwd", "sla_sparse_bwd", "sla_linear_state", "sla_linear_state_static", "sla_fwd", "sla_fwd_gather", "sla_enable_peer_access", "sla_ipc_export", "sla_ipc_open", "sla_ipc_close", "sla_fwd_prepare", "sla_bwd", "sla_bwd_saved",
     "sage_sla_fwd", "sage_sla_fwd_gather", "sage_sla_prepare",
 )
 
@@ -104,6 +104,8 @@ def _load() -> C.CDLL:
     lib.sla_bwd.restype = C.c_int
     lib.sla_bwd.argtypes = [sp, vp, vp, vp, vp, f32p, vp, i32p, i32p, i32p, f32p, vp, vp, vp, vp, f32p, f32p,
                             vp, C.c_size_t, vp]
+    lib.sla_bwd_saved.restype = C.c_int
+    lib.sla_bwd_saved.argtypes = lib.sla_bwd.argtypes[:-3] + [vp, C.c_size_t, vp, C.c_size_t, vp]
     lib.sage_sla_prepare.restype = C.c_int
     lib.sage_sla_prepare.argtypes = [sp, vp, vp, vp, f32p, f32p, vp, vp, C.c_size_t, vp]
     lib.sage_sla_fwd_gather.restype = C.c_int

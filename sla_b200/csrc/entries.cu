@@ -301,11 +301,14 @@ static int sparse_bwd_impl(const sla_shape* s, const void* q, const void* k, con
 }
 
 // Backward of sla_fwd with SLA_FLAG_LINEAR_UNSELECTED (algebra: linear_bwd_unselected.cu). `base` is the workspace of
-// sla_bwd: the all-token regions, the sparse backward's, then ws_bwd_unselected; its 16-bit W has been written.
+// sla_bwd: the all-token regions, the sparse backward's, then ws_bwd_unselected; its 16-bit W has been written. `fwd_ub`:
+// the forward's {phi(q), phi(k), C_num, C_den} (ws_unselected) where the caller kept them, else NULL and they are
+// computed again.
 static int bwd_unselected(const sla_shape* s, const void* q, const void* k, const void* v, const void* o_s,
                           const float* lse, const void* d_o, const int32_t* lut, const int32_t* col_offsets,
                           const int32_t* col_index, const float* w, const void* lin_state, void* dq, void* dk,
-                          void* dv, float* dw, float* dbias, unsigned char* base, cudaStream_t st) {
+                          void* dv, float* dw, float* dbias, unsigned char* base, const unsigned char* fwd_ub,
+                          cudaStream_t st) {
   const WsBwd wb = ws_bwd(s);
   unsigned char* sparse_ws = base + wb.total;
   unsigned char* ub = sparse_ws + ws_sparse_bwd(s).total;
@@ -313,18 +316,25 @@ static int bwd_unselected(const sla_shape* s, const void* q, const void* k, cons
   const int nb = ceil_div(s->L, s->BLKK), Lpad = ceil_div(s->L, 128) * 128;
   const size_t bh = size_t(s->B) * s->H;
   int rc;
-  // the forward's intermediates again: phi(q), phi(k), and the selected blocks' share C_num, C_den
-  if ((rc = run_feature_map(s, q, ub + wu.phiq, st)) != SLA_OK) return rc;
-  if ((rc = run_feature_map(s, k, ub + wu.phik, st)) != SLA_OK) return rc;
-  FwdParams pc = make_fwd(s, ub + wu.phiq, ub + wu.phik, v, lut, ub + wu.cnum, nullptr,
-                          reinterpret_cast<float*>(ub + wu.cden), nullptr, nullptr);
-  pc.plain = 1;
-  if ((rc = run_sparse_fwd_tc(s, pc, st)) != SLA_OK) return rc;
+  const WsUnselected wf = ws_unselected(s);
+  const void* phiq = fwd_ub ? fwd_ub + wf.phiq : ub + wu.phiq;
+  const void* phik = fwd_ub ? fwd_ub + wf.phik : ub + wu.phik;
+  const void* cnum = fwd_ub ? fwd_ub + wf.cnum : ub + wu.cnum;
+  const float* cden = reinterpret_cast<const float*>(fwd_ub ? fwd_ub + wf.cden : ub + wu.cden);
+  if (!fwd_ub) {
+    // the forward's intermediates again: phi(q), phi(k), and the selected blocks' share C_num, C_den
+    if ((rc = run_feature_map(s, q, ub + wu.phiq, st)) != SLA_OK) return rc;
+    if ((rc = run_feature_map(s, k, ub + wu.phik, st)) != SLA_OK) return rc;
+    FwdParams pc = make_fwd(s, phiq, phik, v, lut, ub + wu.cnum, nullptr, reinterpret_cast<float*>(ub + wu.cden), nullptr,
+                            nullptr);
+    pc.plain = 1;
+    if ((rc = run_sparse_fwd_tc(s, pc, st)) != SLA_OK) return rc;
+  }
   // row pass: -dN, dden, the all-token part of dphi_q (into dq), and the partials of G, dz, db, G2
   SLA_CUDA_OK(cudaMemsetAsync(ub + wu.stats, 0, bh * Lpad * sizeof(float2), st));
   UnselBwdParams up;
-  up.phiq = ub + wu.phiq; up.d_o = d_o; up.cnum = ub + wu.cnum;
-  up.cden = reinterpret_cast<const float*>(ub + wu.cden);
+  up.phiq = phiq; up.d_o = d_o; up.cnum = cnum;
+  up.cden = cden;
   up.lin_state = lin_state; up.wbits = base + wb.wbits;
   up.dn_neg = ub + wu.dn_neg; up.dphi = dq;
   up.stats = reinterpret_cast<float2*>(ub + wu.stats);
@@ -346,7 +356,7 @@ static int bwd_unselected(const sla_shape* s, const void* q, const void* k, cons
   // the product without softmax over the selected blocks, on (phi(q), phi(k), v) with dO = -dN, delta = dden:
   // dq += dS phi(k) (still a gradient of phi(q)); dk = phi'(k)(v dH^T + dz + dS^T phi(q)); dv = phi(k) dH + P^T dO
   BwdParams bp;
-  bp.q = ub + wu.phiq; bp.k = ub + wu.phik; bp.v = v; bp.o_s = nullptr; bp.d_o = ub + wu.dn_neg; bp.lse = nullptr;
+  bp.q = phiq; bp.k = phik; bp.v = v; bp.o_s = nullptr; bp.d_o = ub + wu.dn_neg; bp.lse = nullptr;
   bp.delta = nullptr; bp.lut = lut; bp.col_offsets = col_offsets; bp.col_index = col_index;
   bp.dq = dq; bp.dk = dk; bp.dv = dv;
   bp.L = s->L; bp.mb = ceil_div(s->L, s->BLKQ); bp.nb = nb; bp.topk = s->topk;
@@ -354,7 +364,7 @@ static int bwd_unselected(const sla_shape* s, const void* q, const void* k, cons
   bp.lin_dh = lp.dh; bp.lin_dz = lp.dz; bp.plain = 1;
   bp.order = lp.order;
   if ((rc = run_sparse_bwd_tc(s, bp, ub + wu.stats, st)) != SLA_OK) return rc;
-  if ((rc = run_feature_map_bwd(s, ub + wu.phiq, dq, st)) != SLA_OK) return rc;   // dq = phi'(q) dphi_q
+  if ((rc = run_feature_map_bwd(s, phiq, dq, st)) != SLA_OK) return rc;   // dq = phi'(q) dphi_q
   // the softmax branch adds its dq, dk, dv
   return sparse_bwd_impl(s, q, k, v, o_s, lse, d_o, lut, col_offsets, col_index, dq, dk, dv, sparse_ws, 1, st,
                          nullptr, nullptr, true);
@@ -374,10 +384,10 @@ int sla_sparse_bwd(const sla_shape* s, const void* q, const void* k, const void*
                          static_cast<unsigned char*>(ws), 0, static_cast<cudaStream_t>(stream));
 }
 
-int sla_bwd(const sla_shape* s, const void* q, const void* k, const void* v, const void* o_s, const float* lse,
-            const void* d_o, const int32_t* lut, const int32_t* col_offsets, const int32_t* col_index,
-            const float* w, const void* lin_state, void* dq, void* dk, void* dv, float* dw, float* dbias,
-            void* ws, size_t ws_bytes, sla_stream_t stream) {
+static int bwd_impl(const sla_shape* s, const void* q, const void* k, const void* v, const void* o_s, const float* lse,
+                    const void* d_o, const int32_t* lut, const int32_t* col_offsets, const int32_t* col_index,
+                    const float* w, const void* lin_state, void* dq, void* dk, void* dv, float* dw, float* dbias,
+                    void* ws, size_t ws_bytes, const unsigned char* fwd_ub, sla_stream_t stream) {
   const bool linear_only = s && (s->flags & SLA_FLAG_LINEAR_ONLY) != 0;
   if (!q || !k || !v || !d_o || !dq || !dk || !dv || !ws) return SLA_ERR_NULL;
   if (!linear_only && (!o_s || !lse || !lut || !col_offsets || !col_index)) return SLA_ERR_NULL;
@@ -399,7 +409,7 @@ int sla_bwd(const sla_shape* s, const void* q, const void* k, const void* v, con
   if (s->flags & SLA_FLAG_LINEAR_UNSELECTED) {
     if (legacy || linear_only || !sparse_bwd_tc_fits(s) || !sparse_fwd_tc_fits(s)) return SLA_ERR_UNSUPPORTED;
     return bwd_unselected(s, q, k, v, o_s, lse, d_o, lut, col_offsets, col_index, w, lin_state, dq, dk, dv, dw,
-                          dbias, base, st);
+                          dbias, base, fwd_ub, st);
   }
   LinBwdParams lp;
   lp.q = q; lp.k = k; lp.v = v; lp.d_o = d_o; lp.lin_state = lin_state; lp.wbits = base + wb.wbits; lp.w = w;
@@ -422,6 +432,36 @@ int sla_bwd(const sla_shape* s, const void* q, const void* k, const void* v, con
   if (rc != SLA_OK || linear_only) return rc;
   return sparse_bwd_impl(s, q, k, v, o_s, lse, d_o, lut, col_offsets, col_index, dq, dk, dv, sparse_ws, 1, st,
                          fuse_kv ? lp.dh : nullptr, fuse_kv ? lp.dz : nullptr, fuse_kv);
+}
+
+int sla_bwd(const sla_shape* s, const void* q, const void* k, const void* v, const void* o_s, const float* lse,
+            const void* d_o, const int32_t* lut, const int32_t* col_offsets, const int32_t* col_index,
+            const float* w, const void* lin_state, void* dq, void* dk, void* dv, float* dw, float* dbias,
+            void* ws, size_t ws_bytes, sla_stream_t stream) {
+  if (!s) return SLA_ERR_NULL;
+  sla_shape plain = *s;
+  plain.flags &= ~SLA_FLAG_FWD_SAVED;
+  return bwd_impl(&plain, q, k, v, o_s, lse, d_o, lut, col_offsets, col_index, w, lin_state, dq, dk, dv, dw, dbias, ws,
+                  ws_bytes, nullptr, stream);
+}
+
+int sla_bwd_saved(const sla_shape* s, const void* q, const void* k, const void* v, const void* o_s, const float* lse,
+                  const void* d_o, const int32_t* lut, const int32_t* col_offsets, const int32_t* col_index,
+                  const float* w, const void* lin_state, void* dq, void* dk, void* dv, float* dw, float* dbias,
+                  const void* fwd_ws, size_t fwd_ws_bytes, void* ws, size_t ws_bytes, sla_stream_t stream) {
+  if (!s || !fwd_ws) return SLA_ERR_NULL;
+  if (!(s->flags & SLA_FLAG_LINEAR_UNSELECTED) || (s->flags & (SLA_FLAG_SPARSE_ONLY | SLA_FLAG_LINEAR_ONLY)))
+    return SLA_ERR_UNSUPPORTED;
+  int rc = check_common(s);
+  if (rc != SLA_OK) return rc;
+  if (!aligned16(fwd_ws)) return SLA_ERR_BAD_ALIGN;
+  if (fwd_ws_bytes < ws_fwd_total(s)) return SLA_ERR_WS_TOO_SMALL;
+  sla_shape saved = *s;
+  saved.flags |= SLA_FLAG_FWD_SAVED;
+  const unsigned char* fwd_ub =
+      static_cast<const unsigned char*>(fwd_ws) + ws_linear_state(s).total + ws_fwd_extra(s);
+  return bwd_impl(&saved, q, k, v, o_s, lse, d_o, lut, col_offsets, col_index, w, lin_state, dq, dk, dv, dw, dbias, ws,
+                  ws_bytes, fwd_ub, stream);
 }
 
 }  // extern "C"

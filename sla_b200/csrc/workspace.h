@@ -135,7 +135,7 @@ inline WsSparseBwd ws_sparse_bwd(const sla_shape* s) {
 
 // ---- backward of the "unselected" linear scope (behind the two regions above) ----
 struct WsBwdUnselected {
-  size_t phiq, phik, cnum, dn_neg;   // 16-bit [BH][L][D]: phi(q), phi(k), C_num (recomputed), -dN
+  size_t phiq, phik, cnum, dn_neg;   // 16-bit [BH][L][D]: phi(q), phi(k), C_num (recomputed unless saved), -dN
   size_t cden;                       // fp32 [BH][L]
   size_t stats;                      // float2 [BH][Lpad] {unused, dden}
   size_t g_partial;                  // fp32 [BH][NCH][2*D*D + 2*D]
@@ -149,11 +149,14 @@ inline WsBwdUnselected ws_bwd_unselected(const sla_shape* s) {
   const size_t rec = 2 * size_t(s->D) * s->D + 2 * s->D;
   const int nch = ws_bwd(s).nch;
   size_t o = 0;
-  w.phiq = o;      o += ws_round(n * s->D * 2);
-  w.phik = o;      o += ws_round(n * s->D * 2);
-  w.cnum = o;      o += ws_round(n * s->D * 2);
+  w.phiq = w.phik = w.cnum = w.cden = 0;
+  if (!(s->flags & SLA_FLAG_FWD_SAVED)) {      // else they are read from the forward's workspace
+    w.phiq = o;      o += ws_round(n * s->D * 2);
+    w.phik = o;      o += ws_round(n * s->D * 2);
+    w.cnum = o;      o += ws_round(n * s->D * 2);
+    w.cden = o;      o += ws_round(n * 4);
+  }
   w.dn_neg = o;    o += ws_round(n * s->D * 2);
-  w.cden = o;      o += ws_round(n * 4);
   w.stats = o;     o += ws_round(bh * lpad * 8);
   w.g_partial = o; o += ws_round(bh * nch * rec * 4);
   w.g_sum = o;     o += ws_round(bh * rec * 4);

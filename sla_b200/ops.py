@@ -334,24 +334,33 @@ class _SLAFused(torch.autograd.Function):
                               _p(lse), _p(lin_state), _p(ws), ws.numel(), _stream(q)))
         _check_device()
         if need_grad:
-            ctx.save_for_backward(q, k, v, o_s, lse, lin_state, weight, bm.lut, bm.col_offsets, bm.col_index)
+            # the "unselected" scope's backward reads phi(q), phi(k) and the selected blocks' share from the workspace
+            kept = (ws,) if impl_flags & _lib.FLAG_LINEAR_UNSELECTED else ()
+            ctx.save_for_backward(q, k, v, o_s, lse, lin_state, weight, bm.lut, bm.col_offsets, bm.col_index, *kept)
             ctx.sla_shape = shape
+            ctx.feature = feature
             ctx.has_bias = bias is not None
         return o
 
     @staticmethod
     def backward(ctx, d_o):
-        q, k, v, o_s, lse, lin_state, weight, lut, co, ci = ctx.saved_tensors
+        q, k, v, o_s, lse, lin_state, weight, lut, co, ci, *kept = ctx.saved_tensors
         shape = ctx.sla_shape
         d_o = d_o.contiguous()
         D = shape.D
         dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
         dw = torch.empty((D, D), dtype=torch.float32, device=q.device)
         db = torch.empty((D,), dtype=torch.float32, device=q.device)
+        if kept:
+            shape = make_shape(shape.B, shape.H, shape.L, D, shape.BLKQ, shape.BLKK, shape.topk, q.dtype, ctx.feature,
+                               flags=shape.flags | _lib.FLAG_FWD_SAVED)
         ws = _workspace(shape, _lib.OP_BWD, q.device)
-        check(lib.sla_bwd(C.byref(shape), _p(q), _p(k), _p(v), _p(o_s), _p(lse), _p(d_o), _p(lut), _p(co), _p(ci),
-                          _p(weight), _p(lin_state), _p(dq), _p(dk), _p(dv), _p(dw), _p(db), _p(ws), ws.numel(),
-                          _stream(q)))
+        args = (C.byref(shape), _p(q), _p(k), _p(v), _p(o_s), _p(lse), _p(d_o), _p(lut), _p(co), _p(ci), _p(weight),
+                _p(lin_state), _p(dq), _p(dk), _p(dv), _p(dw), _p(db))
+        if kept:
+            check(lib.sla_bwd_saved(*args, _p(kept[0]), kept[0].numel(), _p(ws), ws.numel(), _stream(q)))
+        else:
+            check(lib.sla_bwd(*args, _p(ws), ws.numel(), _stream(q)))
         _check_device()
         return dq, dk, dv, dw, (db if ctx.has_bias else None), None, None, None, None, None, None, None, None, None
 

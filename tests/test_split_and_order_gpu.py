@@ -38,6 +38,34 @@ def test_tile_order_leaves_the_gradients_alone(L, D, BLKQ, heads):
             assert torch.equal(a[:, h], b[:, 0])
 
 
+@pytest.mark.parametrize("L,D,BLKQ,feature", [(777, 64, 64, "relu"), (1500, 128, 128, "softmax")])
+def test_saved_workspace_backward_equals_the_recomputing_one(L, D, BLKQ, feature):
+    m = sla_b200.SparseLinearAttention(D, 0.25, feature, BLKQ, 64, linear_scope="unselected").cuda()
+    with torch.no_grad():
+        m.proj_l.weight.copy_(_randn((D, D), 5, torch.float32) * 0.05)
+    q, k, v, do = (_randn((2, 2, L, D), 20 + i) for i in range(4))
+    ts = [t.clone().requires_grad_(True) for t in (q, k, v)]
+    m(*ts).backward(do)
+
+    bm = ops.block_map(q, k, 0.25, BLKQ, 64, want_cols=True)
+    shape = ops.make_shape(2, 2, L, D, BLKQ, 64, bm.topk, q.dtype, feature, flags=m.impl_flags)
+    o, o_s, lse = torch.empty_like(q), torch.empty_like(q), torch.empty(q.shape[:-1], device="cuda")
+    state = torch.empty((2, 2, 2 * D * D + D), dtype=q.dtype, device="cuda")
+    w, b, p = m.proj_l.weight.detach(), m.proj_l.bias.detach(), ops._p
+    ws = ops._workspace(shape, _lib.OP_FWD, q.device)
+    st = ops._stream(q)
+    _lib.check(_lib.lib.sla_fwd(C.byref(shape), p(q), p(k), p(v), p(bm.lut), p(w), p(b), p(o), p(o_s), p(lse), p(state),
+                                p(ws), ws.numel(), st))
+    out = [torch.empty_like(q) for _ in range(3)]
+    dw, db = torch.empty((D, D), device="cuda"), torch.empty((D,), device="cuda")
+    ws = ops._workspace(shape, _lib.OP_BWD, q.device)
+    _lib.check(_lib.lib.sla_bwd(C.byref(shape), p(q), p(k), p(v), p(o_s), p(lse), p(do), p(bm.lut), p(bm.col_offsets),
+                                p(bm.col_index), p(w), p(state), *(p(t) for t in out), p(dw), p(db), p(ws), ws.numel(), st))
+    for a, t in zip(out, ts):
+        assert torch.equal(a, t.grad)
+    assert torch.equal(dw, m.proj_l.weight.grad) and torch.equal(db, m.proj_l.bias.grad)
+
+
 def test_first_call_of_a_thread_may_be_a_backward():
     """A new process, whose autograd thread has made no CUDA call when the backward encodes its tensor maps."""
     code = """
