@@ -188,9 +188,7 @@ static int fwd_impl(const sla_shape* s, const void* q, const void* k, const void
     rc = run_sparse_fwd_tc(s, ps, st);
     if (rc == SLA_ERR_BAD_SHAPE) return SLA_ERR_UNSUPPORTED;   // this scope has no mma.sync path
     if (rc != SLA_OK) return rc;
-    rc = run_feature_map(s, q, ub + wu.phiq, st);
-    if (rc != SLA_OK) return rc;
-    rc = run_feature_map(s, k, ub + wu.phik, st);
+    rc = run_feature_maps(s, q, ub + wu.phiq, k, ub + wu.phik, st);
     if (rc != SLA_OK) return rc;
     FwdParams pc = make_fwd(s, ub + wu.phiq, ub + wu.phik, v, lut, ub + wu.cnum, nullptr,
                             reinterpret_cast<float*>(ub + wu.cden), nullptr, nullptr);
@@ -323,8 +321,7 @@ static int bwd_unselected(const sla_shape* s, const void* q, const void* k, cons
   const float* cden = reinterpret_cast<const float*>(fwd_ub ? fwd_ub + wf.cden : ub + wu.cden);
   if (!fwd_ub) {
     // the forward's intermediates again: phi(q), phi(k), and the selected blocks' share C_num, C_den
-    if ((rc = run_feature_map(s, q, ub + wu.phiq, st)) != SLA_OK) return rc;
-    if ((rc = run_feature_map(s, k, ub + wu.phik, st)) != SLA_OK) return rc;
+    if ((rc = run_feature_maps(s, q, ub + wu.phiq, k, ub + wu.phik, st)) != SLA_OK) return rc;
     FwdParams pc = make_fwd(s, phiq, phik, v, lut, ub + wu.cnum, nullptr, reinterpret_cast<float*>(ub + wu.cden), nullptr,
                             nullptr);
     pc.plain = 1;

@@ -91,7 +91,7 @@ int run_linear_bwd_reductions(const sla_shape* s, const LinBwdParams& p, cudaStr
 int convert_proj(const sla_shape* s, const float* w, const float* bias, void* out, cudaStream_t st);
 int run_sparse_fwd_mma(const sla_shape* s, const FwdParams& p, bool lin, cudaStream_t st);
 int run_sparse_fwd_tc(const sla_shape* s, const FwdParams& p, cudaStream_t st);
-int run_feature_map(const sla_shape* s, const void* x, void* out, cudaStream_t st);
+int run_feature_maps(const sla_shape* s, const void* q, void* phiq, const void* k, void* phik, cudaStream_t st);
 int run_linear_readout_unselected(const sla_shape* s, const FwdParams& p, const void* cnum, const float* cden,
                                   cudaStream_t st);
 int run_state_proj(const sla_shape* s, void* lin_state, const void* wbits, cudaStream_t st);

@@ -15,64 +15,85 @@
 
 namespace sla {
 
-// out = phi(x) rounded to T, row by row (core.py:90-91). One warp per row.
+// out = phi(x) rounded to T, row by row (core.py:90-91), for q (y = 0) and k (y = 1) in one launch. A row is D / 8 lanes
+// of 16 bytes and a lane has kMapRows rows in flight: the pass is bound by DRAM, and one 8-byte load per lane and row
+// left it at half of the copy bandwidth.
+constexpr int kMapRows = 4;
+
 template <typename T, int D, int FEAT>
-__global__ void __launch_bounds__(256) feature_map_kernel(const T* __restrict__ x, T* __restrict__ out,
-                                                          long long rows) {
-  constexpr int EPL = D / 32;
-  const long long r = static_cast<long long>(blockIdx.x) * 8 + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  if (r >= rows) return;
-  float v[EPL];
-  const T* src = x + r * D + lane * EPL;
+__global__ void __launch_bounds__(256) feature_map_kernel(const T* __restrict__ q, T* __restrict__ phiq,
+                                                          const T* __restrict__ k, T* __restrict__ phik, long long rows) {
+  constexpr int TPR = D / 8, RPP = 256 / TPR;        // lanes per row, rows per pass
+  const T* x = blockIdx.y == 0 ? q : k;
+  T* out = blockIdx.y == 0 ? phiq : phik;
+  const int c = (threadIdx.x % TPR) * 8;
+  const long long r0 = static_cast<long long>(blockIdx.x) * (RPP * kMapRows) + threadIdx.x / TPR;
+  uint4 raw[kMapRows];
 #pragma unroll
-  for (int e = 0; e < EPL; e += 2) {
-    float2 f = Elem<T>::unpack2(*reinterpret_cast<const uint32_t*>(src + e));
-    v[e] = f.x; v[e + 1] = f.y;
+  for (int u = 0; u < kMapRows; ++u) {
+    const long long r = r0 + u * RPP;
+    raw[u] = r < rows ? *reinterpret_cast<const uint4*>(x + r * D + c) : make_uint4(0u, 0u, 0u, 0u);
   }
-  if (FEAT == SLA_PHI_SOFTMAX) {
-    float mx = v[0];
 #pragma unroll
-    for (int e = 1; e < EPL; ++e) mx = fmaxf(mx, v[e]);
-    mx = warp_max(mx);
-    float s = 0.f;
+  for (int u = 0; u < kMapRows; ++u) {
+    const long long r = r0 + u * RPP;
+    uint32_t w[4] = {raw[u].x, raw[u].y, raw[u].z, raw[u].w};
+    float v[8];
 #pragma unroll
-    for (int e = 0; e < EPL; ++e) { v[e] = __expf(v[e] - mx); s += v[e]; }
-    s = 1.f / warp_sum(s);
+    for (int i = 0; i < 4; ++i) {
+      const float2 f = Elem<T>::unpack2(w[i]);
+      v[2 * i] = f.x; v[2 * i + 1] = f.y;
+    }
+    if (FEAT == SLA_PHI_SOFTMAX) {
+      float mx = v[0];
 #pragma unroll
-    for (int e = 0; e < EPL; ++e) v[e] *= s;
-  } else if (FEAT == SLA_PHI_RELU) {
+      for (int e = 1; e < 8; ++e) mx = fmaxf(mx, v[e]);
 #pragma unroll
-    for (int e = 0; e < EPL; ++e) v[e] = fmaxf(v[e], 0.f);
-  } else {
+      for (int o = 1; o < TPR; o <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+      float sm = 0.f;
 #pragma unroll
-    for (int e = 0; e < EPL; ++e) v[e] = v[e] > 0.f ? v[e] + 1.f : __expf(v[e]);
+      for (int e = 0; e < 8; ++e) { v[e] = __expf(v[e] - mx); sm += v[e]; }
+#pragma unroll
+      for (int o = 1; o < TPR; o <<= 1) sm += __shfl_xor_sync(0xffffffffu, sm, o);
+      sm = 1.f / sm;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) v[e] *= sm;
+    } else if (FEAT == SLA_PHI_RELU) {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) v[e] = fmaxf(v[e], 0.f);
+    } else {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) v[e] = v[e] > 0.f ? v[e] + 1.f : __expf(v[e]);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) w[i] = Elem<T>::pack2(v[2 * i], v[2 * i + 1]);
+    if (r < rows) *reinterpret_cast<uint4*>(out + r * D + c) = make_uint4(w[0], w[1], w[2], w[3]);
   }
-  T* dst = out + r * D + lane * EPL;
-#pragma unroll
-  for (int e = 0; e < EPL; e += 2) *reinterpret_cast<uint32_t*>(dst + e) = Elem<T>::pack2(v[e], v[e + 1]);
 }
 
 template <typename T, int D>
-static int feature_map_typed(const sla_shape* s, const T* x, T* out, cudaStream_t st) {
+static int feature_map_typed(const sla_shape* s, const T* q, T* phiq, const T* k, T* phik, cudaStream_t st) {
   const long long rows = static_cast<long long>(s->B) * s->H * s->L;
-  const unsigned grid = static_cast<unsigned>((rows + 7) / 8);
+  constexpr int per = 256 / (D / 8) * kMapRows;
+  const dim3 grid(static_cast<unsigned>((rows + per - 1) / per), 2);
   switch (s->feature_map) {
-    case SLA_PHI_SOFTMAX: feature_map_kernel<T, D, SLA_PHI_SOFTMAX><<<grid, 256, 0, st>>>(x, out, rows); break;
-    case SLA_PHI_RELU: feature_map_kernel<T, D, SLA_PHI_RELU><<<grid, 256, 0, st>>>(x, out, rows); break;
-    default: feature_map_kernel<T, D, SLA_PHI_ELU><<<grid, 256, 0, st>>>(x, out, rows); break;
+    case SLA_PHI_SOFTMAX: feature_map_kernel<T, D, SLA_PHI_SOFTMAX><<<grid, 256, 0, st>>>(q, phiq, k, phik, rows); break;
+    case SLA_PHI_RELU: feature_map_kernel<T, D, SLA_PHI_RELU><<<grid, 256, 0, st>>>(q, phiq, k, phik, rows); break;
+    default: feature_map_kernel<T, D, SLA_PHI_ELU><<<grid, 256, 0, st>>>(q, phiq, k, phik, rows); break;
   }
   SLA_LAUNCH_OK();
   return SLA_OK;
 }
 
-int run_feature_map(const sla_shape* s, const void* x, void* out, cudaStream_t st) {
+int run_feature_maps(const sla_shape* s, const void* q, void* phiq, const void* k, void* phik, cudaStream_t st) {
   if (s->dtype == SLA_BF16) {
     using T = __nv_bfloat16;
-    return s->D == 64 ? feature_map_typed<T, 64>(s, (const T*)x, (T*)out, st) : feature_map_typed<T, 128>(s, (const T*)x, (T*)out, st);
+    return s->D == 64 ? feature_map_typed<T, 64>(s, (const T*)q, (T*)phiq, (const T*)k, (T*)phik, st)
+                      : feature_map_typed<T, 128>(s, (const T*)q, (T*)phiq, (const T*)k, (T*)phik, st);
   }
   using T = __half;
-  return s->D == 64 ? feature_map_typed<T, 64>(s, (const T*)x, (T*)out, st) : feature_map_typed<T, 128>(s, (const T*)x, (T*)out, st);
+  return s->D == 64 ? feature_map_typed<T, 64>(s, (const T*)q, (T*)phiq, (const T*)k, (T*)phik, st)
+                    : feature_map_typed<T, 128>(s, (const T*)q, (T*)phiq, (const T*)k, (T*)phik, st);
 }
 
 // 64 query rows per CTA, one warp per 16 rows: phi(q) rows (already mapped, `p.q`), H, C_num, C_den in;
@@ -175,7 +196,7 @@ static int readout_unselected_typed(const sla_shape* s, const FwdParams& p, cons
   return SLA_OK;
 }
 
-// p.q must hold phi(q) (run_feature_map), p.o_s the sparse branch's output, p.lin_state H and z.
+// p.q must hold phi(q) (run_feature_maps), p.o_s the sparse branch's output, p.lin_state H and z.
 int run_linear_readout_unselected(const sla_shape* s, const FwdParams& p, const void* cnum, const float* cden,
                                   cudaStream_t st) {
   if (s->dtype == SLA_BF16)
