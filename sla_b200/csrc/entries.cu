@@ -129,9 +129,10 @@ int sla_fwd_prepare(const sla_shape* s, const void* k, const void* v, const floa
   unsigned char* base = static_cast<unsigned char*>(ws);
   void* wbits = base + wl.total;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  rc = convert_proj(s, w, bias, wbits, st);
+  ProjConvert proj;
+  rc = start_convert_proj(s, w, bias, wbits, &proj, st);
   if (rc != SLA_OK) return rc;
-  rc = run_linear_state(s, k, v, lin_state, reinterpret_cast<float*>(base + wl.partial), wl.nch, wl.rows, st);
+  rc = run_linear_state(s, k, v, lin_state, reinterpret_cast<float*>(base + wl.partial), wl.nch, wl.rows, st, proj);
   if (rc != SLA_OK) return rc;
   return run_state_proj(s, lin_state, wbits, st);
 }
@@ -170,9 +171,10 @@ static int fwd_impl(const sla_shape* s, const void* q, const void* k, const void
   const bool unselected = (s->flags & SLA_FLAG_LINEAR_UNSELECTED) != 0;
   if (unselected && legacy) return SLA_ERR_UNSUPPORTED;
   if (!(s->flags & SLA_FLAG_STATE_READY)) {
-    rc = convert_proj(s, w, bias, wbits, st);
+    ProjConvert proj;
+    rc = start_convert_proj(s, w, bias, wbits, &proj, st);
     if (rc != SLA_OK) return rc;
-    rc = run_linear_state(s, k, v, lin_state, reinterpret_cast<float*>(base + wl.partial), wl.nch, wl.rows, st);
+    rc = run_linear_state(s, k, v, lin_state, reinterpret_cast<float*>(base + wl.partial), wl.nch, wl.rows, st, proj);
     if (rc != SLA_OK) return rc;
     rc = run_state_proj(s, lin_state, wbits, st);
     if (rc != SLA_OK) return rc;
@@ -401,14 +403,16 @@ static int bwd_impl(const sla_shape* s, const void* q, const void* k, const void
     return sparse_bwd_impl(s, q, k, v, o_s, lse, d_o, lut, col_offsets, col_index, dq, dk, dv, sparse_ws, 0, st);
   if (!w || !lin_state || !dw || !dbias) return SLA_ERR_NULL;
   const bool legacy = (s->flags & SLA_FLAG_LEGACY_MMA) != 0;
-  rc = convert_proj(s, w, nullptr, base + wb.wbits, st);
-  if (rc != SLA_OK) return rc;
   if (s->flags & SLA_FLAG_LINEAR_UNSELECTED) {
+    rc = convert_proj(s, w, nullptr, base + wb.wbits, st);     // its row pass reads W
+    if (rc != SLA_OK) return rc;
     if (legacy || linear_only || !sparse_bwd_tc_fits(s) || !sparse_fwd_tc_fits(s)) return SLA_ERR_UNSUPPORTED;
     return bwd_unselected(s, q, k, v, o_s, lse, d_o, lut, col_offsets, col_index, w, lin_state, dq, dk, dv, dw,
                           dbias, base, fwd_ub, st);
   }
   LinBwdParams lp;
+  rc = start_convert_proj(s, w, nullptr, base + wb.wbits, &lp.proj, st);
+  if (rc != SLA_OK) return rc;
   lp.q = q; lp.k = k; lp.v = v; lp.d_o = d_o; lp.lin_state = lin_state; lp.wbits = base + wb.wbits; lp.w = w;
   lp.dq = dq; lp.dk = dk; lp.dv = dv;
   lp.g_sum = reinterpret_cast<float*>(base + wb.g_sum);

@@ -4,6 +4,7 @@
 #include <stdint.h>
 
 #include "../../include/sla_b200.h"
+#include "common.cuh"
 #include "tile_order.cuh"
 
 namespace sla {
@@ -49,6 +50,26 @@ struct BwdParams {
   TileOrder order;        // tcgen05 path only: order of the dK/dV kernel's last key tiles, order.order made beforehand
 };
 
+// 16-bit copy of proj_l's weight and bias, W then bias
+int convert_proj(const sla_shape* s, const float* w, const float* bias, void* out, cudaStream_t st);
+// The same as one extra row of CTAs of a kernel whose rows are heads (blockIdx.y == row); row < 0: not wanted. Head
+// counts up to the grid limit leave no room for the row: start_convert_proj then launches the kernel of its own.
+struct ProjConvert {
+  const float *w = nullptr, *bias = nullptr;
+  void* out = nullptr;
+  int dd = 0, d = 0, row = -1;
+};
+int start_convert_proj(const sla_shape* s, const float* w, const float* bias, void* out, ProjConvert* merged,
+                       cudaStream_t st);
+#if defined(__CUDACC__)
+template <typename T>
+__device__ inline void convert_proj_element(const ProjConvert& p, int i) {
+  T* out = static_cast<T*>(p.out);
+  if (i < p.dd) out[i] = Elem<T>::from_f(p.w[i]);
+  else if (i < p.dd + p.d) out[i] = Elem<T>::from_f(p.bias ? p.bias[i - p.dd] : 0.f);
+}
+#endif
+
 struct LinBwdParams {
   const void *q, *k, *v, *d_o;
   const void* lin_state;  // H, z (16-bit)
@@ -70,6 +91,7 @@ struct LinBwdParams {
   int g_stride = 0;       // 0: the default record D*D + 2*D
   int has_g2 = 0;
   TileOrder order;        // made by the first reduction kernel on the side when order.order is set
+  ProjConvert proj;       // likewise the 16-bit W that the second one reads
 };
 
 // Row pass of the backward of the "unselected" linear scope.
@@ -88,7 +110,6 @@ int run_linear_bwd_unselected_rows(const sla_shape* s, const UnselBwdParams& p, 
 int run_feature_map_bwd(const sla_shape* s, const void* phi, void* dphi_to_dx, cudaStream_t st);
 int run_linear_bwd_reductions(const sla_shape* s, const LinBwdParams& p, cudaStream_t st);
 
-int convert_proj(const sla_shape* s, const float* w, const float* bias, void* out, cudaStream_t st);
 int run_sparse_fwd_mma(const sla_shape* s, const FwdParams& p, bool lin, cudaStream_t st);
 int run_sparse_fwd_tc(const sla_shape* s, const FwdParams& p, cudaStream_t st);
 int run_feature_maps(const sla_shape* s, const void* q, void* phiq, const void* k, void* phik, cudaStream_t st);
@@ -106,7 +127,7 @@ bool sparse_fwd_tc_fits(const sla_shape* s);
 // softmax variant: fills `stats` ({lse, delta} per row) itself; no-softmax variant (p.plain): reads it
 int run_sparse_bwd_dq_pair(const sla_shape* s, const BwdParams& p, void* stats, int Lpad, cudaStream_t st);
 int run_linear_state(const sla_shape* s, const void* k, const void* v, void* lin_state, float* partial,
-                     int nch, int rows, cudaStream_t st);
+                     int nch, int rows, cudaStream_t st, const ProjConvert& proj = ProjConvert());
 int run_linear_state_static(const sla_shape* s, const void* k, const void* v, void* lin_state, cudaStream_t st);
 int run_k_mean(const sla_shape* s, const void* k, float* partial, float* kmean, cudaStream_t st);
 int run_sparse_bwd_mma(const sla_shape* s, const BwdParams& p, cudaStream_t st);

@@ -172,11 +172,16 @@ __global__ void __launch_bounds__(D / 16 * 32) linear_bwd_q_kernel(LinBwdParams 
 // Per-head reductions. (1) sum the chunk partials (and, in a CTA of its own, the dK/dV kernel's tile order); (2) G -> dH (T), and the head's dW; dz, db copied.
 // ---------------------------------------------------------------------------------------------
 static_assert(kOrderThreads == 256, "the reduction kernel's block size");
+template <typename T>
 __global__ void __launch_bounds__(256) linear_bwd_gsum_kernel(const float* __restrict__ part,
                                                               float* __restrict__ gsum, int nch, int n,
-                                                              TileOrder order) {
+                                                              TileOrder order, ProjConvert proj) {
   pdl_entry();
   const int bh = blockIdx.y;
+  if (bh == proj.row) {              // the row of CTAs behind the heads
+    convert_proj_element<T>(proj, blockIdx.x * 256 + threadIdx.x);
+    return;
+  }
   if (blockIdx.x * 256 >= n) {       // the column of CTAs behind the sums
     if (bh == 0) order_tiles(order);
     return;
@@ -345,8 +350,9 @@ template <typename T, int D>
 static int reductions_typed(const sla_shape* s, const LinBwdParams& p, cudaStream_t st) {
   const int bh = s->B * s->H, dd = D * D;
   const int n = p.g_stride ? p.g_stride : dd + 2 * D;
-  SLA_CUDA_OK(launch_pdl(linear_bwd_gsum_kernel, dim3(ceil_div(n, 256) + (p.order.order ? 1 : 0), bh), dim3(256), 0, st,
-                         static_cast<const float*>(p.g_partial), p.g_sum, p.nch, n, p.order));
+  SLA_CUDA_OK(launch_pdl(linear_bwd_gsum_kernel<T>,
+                         dim3(ceil_div(n, 256) + (p.order.order ? 1 : 0), p.proj.row == bh ? bh + 1 : bh), dim3(256), 0, st,
+                         static_cast<const float*>(p.g_partial), p.g_sum, p.nch, n, p.order, p.proj));
   SLA_LAUNCH_OK();
   auto rk = linear_bwd_reduce_kernel<T, D>;
   SLA_CUDA_OK(cudaFuncSetAttribute(rk, cudaFuncAttributeMaxDynamicSharedMemorySize, 3 * dd * 2));

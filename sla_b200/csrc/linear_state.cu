@@ -157,14 +157,19 @@ __global__ void __launch_bounds__(D / 16 * 32) linear_state_kernel(const T* __re
   linear_state_chunk<T, D, FEAT>(k, v, partial, L, nch, rows, smem);
 }
 
-// n = D*D + D values per head; the head's record is rec_stride elements long (H, z, then room for H W^T)
+// n = D*D + D values per head; the head's record is rec_stride elements long (H, z, then room for H W^T). The row of
+// CTAs behind the heads rounds proj_l's weight and bias (as many values as a head's) to T, which saves a launch.
 template <typename T>
 __global__ void linear_state_reduce_kernel(const float* __restrict__ partial, T* __restrict__ state, int nch,
-                                           int n, int rec_stride) {
+                                           int n, int rec_stride, ProjConvert proj) {
   pdl_wait();
   int bh = blockIdx.y;
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
+  if (bh == proj.row) {
+    convert_proj_element<T>(proj, i);
+    return;
+  }
   const float* p = partial + static_cast<size_t>(bh) * nch * n + i;
   float s = 0.f;
 #pragma unroll 8
@@ -174,13 +179,13 @@ __global__ void linear_state_reduce_kernel(const float* __restrict__ partial, T*
 
 template <typename T, int D>
 static int launch_state(const sla_shape* s, const T* k, const T* v, T* state, float* partial, int nch,
-                        int rows, cudaStream_t st) {
+                        int rows, const ProjConvert& proj, cudaStream_t st) {
   int bh = s->B * s->H;
   dim3 grid(nch, bh);
   const int n = D * D + D;
   auto reduce = [&]() -> int {
-    SLA_CUDA_OK(launch_pdl<false>(linear_state_reduce_kernel<T>, dim3(ceil_div(n, 256), bh), dim3(256), 0, st,
-                                  static_cast<const float*>(partial), state, nch, n, 2 * D * D + D));
+    SLA_CUDA_OK(launch_pdl<false>(linear_state_reduce_kernel<T>, dim3(ceil_div(n, 256), proj.row == bh ? bh + 1 : bh),
+                                  dim3(256), 0, st, static_cast<const float*>(partial), state, nch, n, 2 * D * D + D, proj));
     SLA_LAUNCH_OK();
     return SLA_OK;
   };
@@ -208,15 +213,15 @@ static int launch_state(const sla_shape* s, const T* k, const T* v, T* state, fl
 }
 
 int run_linear_state(const sla_shape* s, const void* k, const void* v, void* lin_state, float* partial, int nch,
-                     int rows, cudaStream_t st) {
+                     int rows, cudaStream_t st, const ProjConvert& proj) {
   if (s->dtype == SLA_BF16) {
     using T = __nv_bfloat16;
-    if (s->D == 64) return launch_state<T, 64>(s, (const T*)k, (const T*)v, (T*)lin_state, partial, nch, rows, st);
-    return launch_state<T, 128>(s, (const T*)k, (const T*)v, (T*)lin_state, partial, nch, rows, st);
+    if (s->D == 64) return launch_state<T, 64>(s, (const T*)k, (const T*)v, (T*)lin_state, partial, nch, rows, proj, st);
+    return launch_state<T, 128>(s, (const T*)k, (const T*)v, (T*)lin_state, partial, nch, rows, proj, st);
   }
   using T = __half;
-  if (s->D == 64) return launch_state<T, 64>(s, (const T*)k, (const T*)v, (T*)lin_state, partial, nch, rows, st);
-  return launch_state<T, 128>(s, (const T*)k, (const T*)v, (T*)lin_state, partial, nch, rows, st);
+  if (s->D == 64) return launch_state<T, 64>(s, (const T*)k, (const T*)v, (T*)lin_state, partial, nch, rows, proj, st);
+  return launch_state<T, 128>(s, (const T*)k, (const T*)v, (T*)lin_state, partial, nch, rows, proj, st);
 }
 
 // ---------------------------------------------------------------------------------------------

@@ -238,9 +238,9 @@ template <typename T>
 __global__ void convert_proj_kernel(const float* __restrict__ w, const float* __restrict__ bias,
                                     T* __restrict__ out, int dd, int d) {
   pdl_wait();
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < dd) out[i] = Elem<T>::from_f(w[i]);
-  else if (i < dd + d) out[i] = Elem<T>::from_f(bias ? bias[i - dd] : 0.f);
+  ProjConvert p;
+  p.w = w; p.bias = bias; p.out = out; p.dd = dd; p.d = d;
+  convert_proj_element<T>(p, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
 int convert_proj(const sla_shape* s, const float* w, const float* bias, void* out, cudaStream_t st) {
@@ -252,6 +252,15 @@ int convert_proj(const sla_shape* s, const float* w, const float* bias, void* ou
     SLA_CUDA_OK(launch_pdl(convert_proj_kernel<__half>, dim3(ceil_div(n, 256)), dim3(256), 0, st, w, bias,
                            static_cast<__half*>(out), dd, s->D));
   SLA_LAUNCH_OK();
+  return SLA_OK;
+}
+
+int start_convert_proj(const sla_shape* s, const float* w, const float* bias, void* out, ProjConvert* merged,
+                       cudaStream_t st) {
+  const int bh = s->B * s->H;
+  if (bh >= 65535) return convert_proj(s, w, bias, out, st);
+  merged->w = w; merged->bias = bias; merged->out = out;
+  merged->dd = s->D * s->D; merged->d = s->D; merged->row = bh;
   return SLA_OK;
 }
 

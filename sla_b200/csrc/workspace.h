@@ -47,8 +47,8 @@ inline WsLinearState ws_linear_state(const sla_shape* s) {
   size_t bh = size_t(s->B) * s->H;
   // The split of a head's rows into chunks fixes the order of the fp32 sums. It depends on L alone, never on
   // B or H, so a (batch, head) unit gives the same bits whatever else is in the batch and however the units are
-  // sharded over GPUs: at most 64 chunks per head, at least 512 rows per chunk.
-  int nch = ws_ceil_div(s->L, 512);
+  // sharded over GPUs: at most 64 chunks per head, at least 256 rows per chunk.
+  int nch = ws_ceil_div(s->L, 256);
   if (nch > 64) nch = 64;
   int rows = (ws_ceil_div(s->L, nch) + 127) / 128 * 128;
   w.rows = rows;
@@ -84,7 +84,7 @@ inline size_t ws_fwd_total(const sla_shape* s) {
 
 // ---- backward ----
 struct WsBwd {
-  size_t wbits;     // 16-bit copy of W [D][D]
+  size_t wbits;     // 16-bit copy of W [D][D], then of the bias (zeros)
   size_t g_partial; // fp32 [BH][NCH][D*D + 2*D]: G, dz, db partials of the linear backward
   size_t dh;        // 16-bit [BH][D*D] dH, then fp32 [BH][D] dz
   size_t dz;
@@ -97,14 +97,14 @@ inline WsBwd ws_bwd(const sla_shape* s) {
   WsBwd w;
   size_t bh = size_t(s->B) * s->H;
   // chunks of the linear backward's row passes: a function of L alone, like ws_linear_state
-  int nch = ws_ceil_div(s->L, 512);
+  int nch = ws_ceil_div(s->L, 256);
   if (nch > 64) nch = 64;
   int rows = (ws_ceil_div(s->L, nch) + 127) / 128 * 128;
   w.rows = rows;
   w.nch = ws_ceil_div(s->L, rows);
   size_t dd = size_t(s->D) * s->D;
   size_t o = 0;
-  w.wbits = o;     o += ws_round(dd * 2);
+  w.wbits = o;     o += ws_round(dd * 2 + s->D * 2);
   w.g_partial = o; o += ws_round(bh * w.nch * (dd + 2 * s->D) * 4);
   w.dh = o;        o += ws_round(bh * dd * 2);
   w.dz = o;        o += ws_round(bh * s->D * 4);
