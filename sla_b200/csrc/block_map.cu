@@ -75,7 +75,7 @@ constexpr int kPoolWarps = 8;
 
 template <typename TIn, int D, bool IS_K>
 __device__ inline void pool_blocks(const TIn* __restrict__ x, const float* __restrict__ kmean,
-                                   TIn* __restrict__ pooled, int L, int blk, int nblk) {
+                                   TIn* __restrict__ pooled, int L, int blk, int nblk, int mean_nch) {
   constexpr int N = VecLoad<TIn>::N;
   constexpr int TPR = D / N;        // lanes per row
   constexpr int RPW = 32 / TPR;     // rows per warp-wide load
@@ -87,8 +87,7 @@ __device__ inline void pool_blocks(const TIn* __restrict__ x, const float* __res
   const int row0 = ib * blk, row1 = min(L, row0 + blk);
   const TIn* base = x + static_cast<size_t>(bh) * L * D + c;
   float mean[N];
-#pragma unroll
-  for (int i = 0; i < N; ++i) mean[i] = IS_K ? kmean[static_cast<size_t>(bh) * D + c + i] : 0.f;
+  if constexpr (IS_K) load_k_mean<TIn, N>(mean, kmean, bh, c, L, mean_nch, D);
   float acc[N];
 #pragma unroll
   for (int i = 0; i < N; ++i) acc[i] = 0.f;
@@ -106,7 +105,7 @@ __device__ inline void pool_blocks(const TIn* __restrict__ x, const float* __res
       }
     } else {
 #pragma unroll
-      for (int i = 0; i < N; ++i) acc[i] += IS_K ? round_to<TIn>(v[i] - mean[i]) : v[i];
+      for (int i = 0; i < N; ++i) if constexpr (IS_K) acc[i] += round_to<TIn>(v[i] - mean[i]); else acc[i] += v[i];
     }
   }
 #pragma unroll
@@ -123,15 +122,15 @@ __device__ inline void pool_blocks(const TIn* __restrict__ x, const float* __res
   }
 }
 
-// z = 0: Q, z = 1: K - mean
+// z = 0: Q, z = 1: K - mean. `kmean`: the column means, or with mean_nch > 0 the chunk sums they are made from
 template <typename TIn, int D>
 __global__ void __launch_bounds__(kPoolWarps * 32) pool_kernel(const TIn* __restrict__ q, const TIn* __restrict__ k,
                                                                const float* __restrict__ kmean,
                                                                TIn* __restrict__ pooled_q, TIn* __restrict__ pooled_k,
-                                                               int L, int blkq, int blkk, int mb, int nb) {
+                                                               int L, int blkq, int blkk, int mb, int nb, int mean_nch) {
   pdl_wait();
-  if (blockIdx.z == 0) pool_blocks<TIn, D, false>(q, nullptr, pooled_q, L, blkq, mb);
-  else pool_blocks<TIn, D, true>(k, kmean, pooled_k, L, blkk, nb);
+  if (blockIdx.z == 0) pool_blocks<TIn, D, false>(q, nullptr, pooled_q, L, blkq, mb, 0);
+  else pool_blocks<TIn, D, true>(k, kmean, pooled_k, L, blkk, nb, mean_nch);
 }
 
 // ---- 4. pooled scores + per-row top-k ----
@@ -474,6 +473,66 @@ __global__ void __launch_bounds__(1024) col_fill_kernel(const int8_t* __restrict
   }
 }
 
+// ---- 6a. offsets and lists in one kernel, for heads whose map is small ----
+// The first column of a CTA starts at the number of set entries in all columns to its left, which the CTA counts
+// itself, and so does it with its own 32 columns before it fills them. That re-reads the map up to nb / 32 times from
+// the L2, so it is for maps of at most kSmallMap bytes a head; it takes the place of a memset, the atomic counts of the
+// selection and the scan, three dependent steps that cost more than the reads there.
+constexpr int kSmallMap = 65536;
+
+__global__ void __launch_bounds__(1024) col_lists_small_kernel(const int8_t* __restrict__ sparse_map,
+                                                               int32_t* __restrict__ col_offsets,
+                                                               int32_t* __restrict__ col_index, int mb, int nb, int topk) {
+  __shared__ int32_t cnt[32][33];   // [warp][column]
+  __shared__ int32_t left[32];
+  pdl_wait();
+  const int bh = blockIdx.y, j0 = blockIdx.x * 32;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int8_t* m = sparse_map + static_cast<size_t>(bh) * mb * nb;
+  const bool have = j0 + lane < nb;
+  int before = 0, own = 0;          // lane: columns lane mod 32 to the left, column j0 + lane; rows warp mod 32
+#pragma unroll 4
+  for (int i = warp; i < mb; i += 32) {
+    const int8_t* row = m + static_cast<size_t>(i) * nb + lane;
+    for (int c = 0; c < j0; c += 32) before += row[c] != 0 ? 1 : 0;
+    own += have && row[j0] != 0 ? 1 : 0;
+  }
+  before = __reduce_add_sync(0xffffffffu, before);
+  if (lane == 0) left[warp] = before;
+  cnt[warp][lane] = own;
+  __syncthreads();
+  // every warp: first position of column `lane`, and of this warp's entries in it. Rows are taken in blocks of
+  // consecutive rows below, so the per-warp counts are made again there.
+  int total = 0;
+#pragma unroll 8
+  for (int w = 0; w < 32; ++w) total += cnt[w][lane];
+  int incl = total;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const int up = __shfl_up_sync(0xffffffffu, incl, d);
+    if (lane >= d) incl += up;
+  }
+  int pos = __reduce_add_sync(0xffffffffu, left[lane]) + incl - total;
+  int32_t* off = col_offsets + static_cast<size_t>(bh) * (nb + 1);
+  if (warp == 0) {
+    if (have) off[j0 + lane] = pos;
+    if (j0 + lane == nb - 1) off[nb] = pos + total;
+  }
+  __syncthreads();
+  // ascending rows: warp w owns rows [w * per, (w + 1) * per)
+  const int per = (mb + 31) / 32, r0 = warp * per, r1 = min(mb, r0 + per);
+  int mine = 0;
+  if (have)
+    for (int i = r0; i < r1; ++i) mine += m[static_cast<size_t>(i) * nb + j0 + lane] != 0 ? 1 : 0;
+  cnt[warp][lane] = mine;
+  __syncthreads();
+  for (int w = 0; w < warp; ++w) pos += cnt[w][lane];
+  int32_t* out = col_index + static_cast<size_t>(bh) * mb * topk;
+  if (have)
+    for (int i = r0; i < r1; ++i)
+      if (m[static_cast<size_t>(i) * nb + j0 + lane] != 0) out[pos++] = i;
+}
+
 // ---- 6b. per-column counts straight from a 0/1 map (for maps not produced by sla_block_map) ----
 __global__ void __launch_bounds__(1024) col_count_kernel(const int8_t* __restrict__ sparse_map,
                                                          int32_t* __restrict__ col_offsets, int mb, int nb) {
@@ -510,11 +569,14 @@ static int launch_block_map(const sla_shape* s, const TIn* q, const TIn* k, int3
 
   SLA_CUDA_OK(launch_pdl<false>(colsum_kernel<TIn, D>, dim3(w.nch, bh), dim3(256), 0, st, k, partial, L, w.nch));
   SLA_LAUNCH_OK();
-  SLA_CUDA_OK(launch_pdl<false>(kmean_finalize_kernel<TIn>, dim3(bh), dim3(D), 0, st, partial, kmean, L, w.nch, D));
-  SLA_LAUNCH_OK();
+  const bool inline_mean = w.nch <= kInlineMeanChunks;
+  if (!inline_mean) {
+    SLA_CUDA_OK(launch_pdl<false>(kmean_finalize_kernel<TIn>, dim3(bh), dim3(D), 0, st, partial, kmean, L, w.nch, D));
+    SLA_LAUNCH_OK();
+  }
   SLA_CUDA_OK(launch_pdl<false>(pool_kernel<TIn, D>, dim3(ceil_div(max(mb, nb), kPoolWarps), bh, 2),
-                                dim3(kPoolWarps * 32), 0, st, q, k, static_cast<const float*>(kmean), pq, pk, L,
-                                s->BLKQ, s->BLKK, mb, nb));
+                                dim3(kPoolWarps * 32), 0, st, q, k, static_cast<const float*>(inline_mean ? partial : kmean),
+                                pq, pk, L, s->BLKQ, s->BLKK, mb, nb, inline_mean ? w.nch : 0));
   SLA_LAUNCH_OK();
   return score_and_select<TIn, D>(s, pq, pk, lut, sparse_map, col_offsets, col_index, st);
 }
@@ -526,14 +588,16 @@ static int score_and_select(const sla_shape* s, const TIn* pq, const TIn* pk, in
   const int bh = s->B * s->H, L = s->L;
   const int mb = ceil_div(L, s->BLKQ), nb = ceil_div(L, s->BLKK);
   const bool want_cols = col_offsets != nullptr && col_index != nullptr;
-  if (want_cols) SLA_CUDA_OK(cudaMemsetAsync(col_offsets, 0, sizeof(int32_t) * size_t(bh) * (nb + 1), st));
+  const bool small = want_cols && static_cast<long long>(mb) * nb <= kSmallMap;
+  int32_t* counts = want_cols && !small ? col_offsets : nullptr;      // where the selection counts per column
+  if (counts) SLA_CUDA_OK(cudaMemsetAsync(col_offsets, 0, sizeof(int32_t) * size_t(bh) * (nb + 1), st));
   if constexpr (sizeof(TIn) == 2) {
     const size_t smem = size_t(kMmaRows) * score_key_stride(nb) * 4;
     if (smem > 200 * 1024) return SLA_ERR_BAD_SHAPE;
     auto kern = score_topk_mma_kernel<TIn, D>;
     SLA_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
     SLA_CUDA_OK(launch_pdl<false>(kern, dim3(ceil_div(mb, kMmaRows), bh), dim3(kMmaWarps * 32), smem, st, pq, pk, lut,
-                                  sparse_map, want_cols ? col_offsets : nullptr, mb, nb, s->topk));
+                                  sparse_map, counts, mb, nb, s->topk));
     SLA_LAUNCH_OK();
   } else {
     // fp32 inputs: the scalar kernel (one sequential fp32 sum per score)
@@ -543,10 +607,14 @@ static int score_and_select(const sla_shape* s, const TIn* pq, const TIn* pk, in
     auto kern = score_topk_kernel<TIn, D>;
     SLA_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
     SLA_CUDA_OK(launch_pdl<false>(kern, dim3(ceil_div(mb, kTopkRows), bh), dim3(kTopkRows * 32), smem, st, pq, pk, lut,
-                                  sparse_map, want_cols ? col_offsets : nullptr, mb, nb, s->topk));
+                                  sparse_map, counts, mb, nb, s->topk));
     SLA_LAUNCH_OK();
   }
-  if (want_cols) {
+  if (small) {
+    SLA_CUDA_OK(launch_pdl<false>(col_lists_small_kernel, dim3(ceil_div(nb, 32), bh), dim3(1024), 0, st,
+                                  static_cast<const int8_t*>(sparse_map), col_offsets, col_index, mb, nb, s->topk));
+    SLA_LAUNCH_OK();
+  } else if (want_cols) {
     SLA_CUDA_OK(launch_pdl<false>(col_scan_kernel, dim3(bh), dim3(1024), 0, st, col_offsets, nb));
     SLA_LAUNCH_OK();
     SLA_CUDA_OK(launch_pdl<false>(col_fill_kernel, dim3(ceil_div(nb, 32), bh), dim3(1024), 0, st,
@@ -558,22 +626,26 @@ static int score_and_select(const sla_shape* s, const TIn* pq, const TIn* pk, in
 }
 
 // Column mean of K per head, rounded to the element type (what k.mean(dim=-2) returns): used by the
-// SageSLA path (SageSLA/core.py:102). partial: fp32 [BH][ceil(L/512)][D]; kmean: fp32 [BH][D].
+// SageSLA path (SageSLA/core.py:102). partial: fp32 [BH][ceil(L/512)][D]; kmean: fp32 [BH][D]. *mean_nch is what
+// load_k_mean takes: 0 and the means in kmean, or the number of chunk sums in `partial` for short sequences.
 template <typename TIn, int D>
-static int k_mean_typed(const sla_shape* s, const TIn* k, float* partial, float* kmean, cudaStream_t st) {
+static int k_mean_typed(const sla_shape* s, const TIn* k, float* partial, float* kmean, int* mean_nch, cudaStream_t st) {
   const int bh = s->B * s->H, nch = ceil_div(s->L, kColsumRows);
   colsum_kernel<TIn, D><<<dim3(nch, bh), 256, 0, st>>>(k, partial, s->L, nch);
   SLA_LAUNCH_OK();
-  kmean_finalize_kernel<TIn><<<bh, D, 0, st>>>(partial, kmean, s->L, nch, D);
-  SLA_LAUNCH_OK();
+  *mean_nch = nch <= kInlineMeanChunks ? nch : 0;
+  if (*mean_nch == 0) {
+    kmean_finalize_kernel<TIn><<<bh, D, 0, st>>>(partial, kmean, s->L, nch, D);
+    SLA_LAUNCH_OK();
+  }
   return SLA_OK;
 }
-int run_k_mean(const sla_shape* s, const void* k, float* partial, float* kmean, cudaStream_t st) {
+int run_k_mean(const sla_shape* s, const void* k, float* partial, float* kmean, int* mean_nch, cudaStream_t st) {
   if (s->dtype == SLA_BF16)
-    return s->D == 64 ? k_mean_typed<__nv_bfloat16, 64>(s, (const __nv_bfloat16*)k, partial, kmean, st)
-                      : k_mean_typed<__nv_bfloat16, 128>(s, (const __nv_bfloat16*)k, partial, kmean, st);
-  return s->D == 64 ? k_mean_typed<__half, 64>(s, (const __half*)k, partial, kmean, st)
-                    : k_mean_typed<__half, 128>(s, (const __half*)k, partial, kmean, st);
+    return s->D == 64 ? k_mean_typed<__nv_bfloat16, 64>(s, (const __nv_bfloat16*)k, partial, kmean, mean_nch, st)
+                      : k_mean_typed<__nv_bfloat16, 128>(s, (const __nv_bfloat16*)k, partial, kmean, mean_nch, st);
+  return s->D == 64 ? k_mean_typed<__half, 64>(s, (const __half*)k, partial, kmean, mean_nch, st)
+                    : k_mean_typed<__half, 128>(s, (const __half*)k, partial, kmean, mean_nch, st);
 }
 
 }  // namespace sla

@@ -62,6 +62,11 @@ __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepc
 __device__ __forceinline__ void pdl_entry() { pdl_wait(); pdl_launch_dependents(); }
 #endif
 
+// Column means of K: for sequences of up to kInlineMeanChunks chunks of kColsumRows rows the kernels that need the mean
+// add the chunks' sums themselves, in the order of the kernel that does it for longer ones, instead of launching that
+// kernel: some loads from the L2 a thread against a launch of 4-5 us of host time.
+constexpr int kInlineMeanChunks = 8;
+
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 inline size_t round256(size_t x) { return (x + 255) & ~size_t(255); }
 inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
@@ -137,6 +142,28 @@ struct Elem<float> {
 template <typename T>
 __device__ inline float round_to(float x) {
   return Elem<T>::to_f(Elem<T>::from_f(x));
+}
+
+// mean of N columns starting at c: from the finished means, or from `nch` chunk sums when nch > 0 (same bits)
+template <typename TIn, int N>
+__device__ inline void load_k_mean(float (&mean)[N], const float* __restrict__ src, int bh, int c, int L, int nch, int D) {
+  if (nch == 0) {
+#pragma unroll
+    for (int i = 0; i < N; ++i) mean[i] = src[static_cast<size_t>(bh) * D + c + i];
+    return;
+  }
+#pragma unroll
+  for (int i = 0; i < N; ++i) mean[i] = 0.f;
+  for (int ch = 0; ch < nch; ++ch) {
+    const float4* p = reinterpret_cast<const float4*>(src + (static_cast<size_t>(bh) * nch + ch) * D + c);
+#pragma unroll
+    for (int i = 0; i < N; i += 4) {
+      const float4 v = p[i / 4];
+      mean[i] += v.x; mean[i + 1] += v.y; mean[i + 2] += v.z; mean[i + 3] += v.w;
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < N; ++i) mean[i] = round_to<TIn>(mean[i] / static_cast<float>(L));
 }
 
 // ---------------------------------------------------------------------------------------------

@@ -18,6 +18,29 @@ def _randn(shape, seed, dtype=torch.bfloat16):
     return torch.randn(shape, generator=g, device="cuda").to(dtype)
 
 
+@pytest.mark.parametrize("L,BLKQ,topk", [
+    (64, 64, 1.0), (2049, 64, 0.2), (2111, 128, 0.5), (16384, 64, 0.05),    # lists in one kernel
+    (16385, 64, 0.05), (32700, 128, 0.03),                                  # counted, scanned, filled
+])
+def test_column_lists_match_the_map(L, BLKQ, topk):
+    q, k = _randn((2, 3, L, 64), 1), _randn((2, 3, L, 64), 2)
+    bm = ops.block_map(q, k, topk, BLKQ, 64, want_map=True, want_cols=True)
+    co, ci = ops.column_lists(bm.sparse_map, L, BLKQ, 64, bm.topk)
+    assert torch.equal(bm.col_offsets, co)
+    assert torch.equal(bm.col_index, ci)
+
+
+@pytest.mark.parametrize("L", [500, 4096, 4097])       # one chunk of K sums, the most that are added inline, one more
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_block_map_at_the_inline_mean_edge(L, dtype):
+    q, k = _randn((1, 2, L, 64), 3, dtype), _randn((1, 2, L, 64), 4, dtype) + 0.5
+    lut = ops.block_map(q, k, 0.25, 64, 64).lut.cpu()
+    score = O.pooled_scores(q.cpu(), k.cpu(), 64, 64)
+    want = O.select_topk(score, lut.shape[-1])
+    _, _, bad = O.lut_rows_equal_up_to_ties(score, lut, want, ulps=2)   # sums of another order: one unit either way
+    assert bad == 0
+
+
 @pytest.mark.parametrize("L,D,BLKQ,heads", [(1000, 64, 64, 24), (2500, 128, 128, 9), (19000, 64, 128, 3)])
 def test_tile_order_leaves_the_gradients_alone(L, D, BLKQ, heads):
     """All heads in one call take the ordered tiles (more than one per SM), a head by itself the sequence order."""
