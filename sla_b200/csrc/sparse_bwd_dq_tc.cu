@@ -357,13 +357,13 @@ sparse_bwd_dq_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_
     if (trc) trc[4] = clock64() - clk0;
     const uint32_t t1 = tmem + lane_addr + COL_T1 + wg * 32, t2 = tmem + lane_addr + COL_T2 + wg * 32;
     for (int pi = 0; ok && pi < n_pairs; ++pi) {
-      if (!mbar_wait(BAR(B_T1), pi & 1, kQErrT1, p.err)) { ok = false; break; }
-      if (*abortp) { ok = false; break; }
-      if (trc && pi == 0) trc[5] = clock64() - clk0;
-      tc_fence_after();
+      // read in front of the wait (a role that gives up sets the error word first, which ends this wait as well)
       const int entry = ulist[2 * pi + ent];
       const bool active = (entry >> (28 + half)) & 1;
       const int valid = L - (entry & 0x0fffffff) * 64;       // keys of this block that exist (kernel.py:157)
+      if (!mbar_wait(BAR(B_T1), pi & 1, kQErrT1, p.err)) { ok = false; break; }
+      if (trc && pi == 0) trc[5] = clock64() - clk0;
+      tc_fence_after();
       uint32_t sv[32];
       tmem_ld_x32(t1, sv);
       tmem_wait_ld();

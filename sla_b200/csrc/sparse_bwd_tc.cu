@@ -352,13 +352,13 @@ sparse_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_co
       const int buf = NB == 2 ? (wg & 1) : j % NB;
       long long* trc = ((warp & 3) == 0 && lane == 0) ? tr : nullptr;
       trace_ev(trc, 2 + ch, j, 0);
+      // the row statistics, there long before the scores, and the entry are waited for in front of the scores (a role
+      // that gives up sets the error word first, which ends these waits as well)
+      const bool active = (ulist[j / SL] >> (28 + half)) & 1;
+      if (!mbar_wait(BAR(B_YF + j % NS), (j / NS) & 1, kBErrYFull, p.err)) { ok = false; break; }
       if (!mbar_wait(BAR(B_T + buf), (j / NB) & 1, kBErrTFull, p.err)) { ok = false; break; }
-      if (*abortp) { ok = false; break; }
       trace_ev(trc, 2 + ch, j, 1);
-      if (!mbar_wait(BAR(B_YF + j % NS), (j / NS) & 1, kBErrYFull, p.err)) { ok = false; break; }  // row stats landed
       tc_fence_after();
-      const int entry = ulist[j / SL];
-      const bool active = (entry >> (28 + half)) & 1;
       const uint32_t t1 = tmem + lane_addr + COL_T + buf * 128 + ch * 32, t2 = t1 + 64;
       const float4* stc = reinterpret_cast<const float4*>(stat_p + (j % NS) * 64 + ch * 32);
       uint32_t pp[16], ds[16];

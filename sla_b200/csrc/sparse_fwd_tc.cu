@@ -119,12 +119,12 @@ sparse_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       mbar_init(BAR(B_E + s), 1);
       mbar_init(BAR(B_KE + s), 1);
       mbar_init(BAR(B_S + s), 1);
-      mbar_init(BAR(B_P + s), 128);
+      mbar_init(BAR(B_P + s), 4);      // one arrival per softmax warp
     }
     mbar_init(BAR(B_PV), 1);
     mbar_init(BAR(B_PV + 1), 1);
     mbar_init(BAR(B_HW), 1);
-    mbar_init(BAR(B_PHI), 128);
+    mbar_init(BAR(B_PHI), 4);
     mbar_init(BAR(B_LIN), 1);
     fence_barrier_init();
     fence_proxy_async_smem();
@@ -298,11 +298,11 @@ sparse_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     float m_true = -INFINITY, m_used = -INFINITY, l = 0.f;
     bool ok = !*abortp;
     for (int j = 0; ok && j < n_ent; ++j) {
-      const int b = j & 1;
+      // read in front of the wait: what follows it up to the load of S is on the critical path of the tile. A role
+      // that gives up sets the error word first, which ends this wait as well.
+      const int b = j & 1, entry = ulist[j];
       if (!mbar_wait(BAR(B_S + b), (j >> 1) & 1, kErrSFull, p.err)) { ok = false; break; }
-      if (*abortp) { ok = false; break; }
       tc_fence_after();
-      const int entry = ulist[j];
       const bool active = BM == 128 || ((entry >> (28 + half)) & 1);
       const uint32_t s_addr = tmem + lane_addr + COL_S + b * 64;
       uint32_t pk[32];
@@ -323,7 +323,7 @@ sparse_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           tmem_st_x32(s_addr, pk);
           tmem_wait_st();
           tc_fence_before();
-          mbar_arrive(BAR(B_P + b));
+          mbar_arrive_warp(BAR(B_P + b), lane);
           continue;
         }
         const int valid = L - (entry & 0x0fffffff) * 64;     // keys of this block that exist (kernel.py:57)
@@ -386,7 +386,7 @@ sparse_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       tmem_st_x32(s_addr, pk);
       tmem_wait_st();
       tc_fence_before();
-      mbar_arrive(BAR(B_P + b));
+      mbar_arrive_warp(BAR(B_P + b), lane);
     }
     if (ok && n_ent > 0) ok = mbar_wait(BAR(B_PV + ((n_ent - 1) & 1)), ((n_ent - 1) >> 1) & 1, kErrPvDone, p.err);
     if (!ok) *abortp = 1;
@@ -522,7 +522,7 @@ sparse_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         }
         fence_proxy_async_smem();
         tc_fence_before();
-        mbar_arrive(BAR(B_PHI));
+        mbar_arrive_warp(BAR(B_PHI), lane);
         asm volatile("bar.sync 1, 128;\n" ::: "memory");     // s_rden of this thread's row was written by another thread
         const float rden = s_rden[row];
         // ---- while the read-out GEMM runs: the sparse branch's own output, staged in the idle V stages ----
