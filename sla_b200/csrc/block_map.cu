@@ -64,7 +64,8 @@ __global__ void kmean_finalize_kernel(const float* __restrict__ partial, float* 
   int bh = blockIdx.x, d = threadIdx.x;
   if (d >= D) return;
   float s = 0.f;
-  for (int c = 0; c < nch; ++c) s += partial[(static_cast<size_t>(bh) * nch + c) * D + d];
+#pragma unroll 16
+  for (int c = 0; c < nch; ++c) s += partial[(static_cast<size_t>(bh) * nch + c) * D + d];   // loads batched, sum in order
   kmean[static_cast<size_t>(bh) * D + d] = round_to<TIn>(s / static_cast<float>(L));
 }
 
@@ -550,6 +551,15 @@ __global__ void __launch_bounds__(1024) col_count_kernel(const int8_t* __restric
   if (lane == 0) col_offsets[static_cast<size_t>(bh) * (nb + 1) + j + 1] = cnt;
 }
 
+static bool col_lists_small(int mb, int nb) { return static_cast<long long>(mb) * nb <= kSmallMap; }
+// Zeroes the per-column counts of the selection. First in the chain of dependent kernels, not between two of them.
+static int clear_counts(const sla_shape* s, int32_t* col_offsets, const int32_t* col_index, cudaStream_t st) {
+  const int mb = ceil_div(s->L, s->BLKQ), nb = ceil_div(s->L, s->BLKK);
+  if (col_offsets != nullptr && col_index != nullptr && !col_lists_small(mb, nb))
+    SLA_CUDA_OK(cudaMemsetAsync(col_offsets, 0, sizeof(int32_t) * size_t(s->B) * s->H * (nb + 1), st));
+  return SLA_OK;
+}
+
 template <typename TIn, int D>
 static int score_and_select(const sla_shape* s, const TIn* pq, const TIn* pk, int32_t* lut, int8_t* sparse_map,
                             int32_t* col_offsets, int32_t* col_index, cudaStream_t st);
@@ -567,6 +577,8 @@ static int launch_block_map(const sla_shape* s, const TIn* q, const TIn* k, int3
   const bool want_cols = col_offsets != nullptr && col_index != nullptr;
   if (want_cols && sparse_map == nullptr) sparse_map = reinterpret_cast<int8_t*>(ws + w.map);
 
+  const int rc = clear_counts(s, col_offsets, col_index, st);
+  if (rc != SLA_OK) return rc;
   SLA_CUDA_OK(launch_pdl<false>(colsum_kernel<TIn, D>, dim3(w.nch, bh), dim3(256), 0, st, k, partial, L, w.nch));
   SLA_LAUNCH_OK();
   const bool inline_mean = w.nch <= kInlineMeanChunks;
@@ -588,9 +600,8 @@ static int score_and_select(const sla_shape* s, const TIn* pq, const TIn* pk, in
   const int bh = s->B * s->H, L = s->L;
   const int mb = ceil_div(L, s->BLKQ), nb = ceil_div(L, s->BLKK);
   const bool want_cols = col_offsets != nullptr && col_index != nullptr;
-  const bool small = want_cols && static_cast<long long>(mb) * nb <= kSmallMap;
-  int32_t* counts = want_cols && !small ? col_offsets : nullptr;      // where the selection counts per column
-  if (counts) SLA_CUDA_OK(cudaMemsetAsync(col_offsets, 0, sizeof(int32_t) * size_t(bh) * (nb + 1), st));
+  const bool small = col_lists_small(mb, nb);
+  int32_t* counts = want_cols && !small ? col_offsets : nullptr;      // zeroed by clear_counts
   if constexpr (sizeof(TIn) == 2) {
     const size_t smem = size_t(kMmaRows) * score_key_stride(nb) * 4;
     if (smem > 200 * 1024) return SLA_ERR_BAD_SHAPE;
@@ -610,7 +621,7 @@ static int score_and_select(const sla_shape* s, const TIn* pq, const TIn* pk, in
                                   sparse_map, counts, mb, nb, s->topk));
     SLA_LAUNCH_OK();
   }
-  if (small) {
+  if (want_cols && small) {
     SLA_CUDA_OK(launch_pdl<false>(col_lists_small_kernel, dim3(ceil_div(nb, 32), bh), dim3(1024), 0, st,
                                   static_cast<const int8_t*>(sparse_map), col_offsets, col_index, mb, nb, s->topk));
     SLA_LAUNCH_OK();
@@ -841,6 +852,8 @@ static int block_map_pooled_typed(const sla_shape* s, const unsigned char* sums,
   TIn* pq = reinterpret_cast<TIn*>(ws + w.pooled_q);
   TIn* pk = reinterpret_cast<TIn*>(ws + w.pooled_k);
   if (col_offsets != nullptr && sparse_map == nullptr) sparse_map = reinterpret_cast<int8_t*>(ws + w.map);
+  const int rc = clear_counts(s, col_offsets, col_index, st);
+  if (rc != SLA_OK) return rc;
   pooled_kmean_kernel<TIn><<<bh, 1024, 0, st>>>(ksum, kmean, s->L, nb, D);
   SLA_LAUNCH_OK();
   pooled_finalize_kernel<TIn><<<dim3(ceil_div(max(mb, nb) * D, 256), bh, 2), 256, 0, st>>>(qsum, ksum, kmean, pq, pk, s->L,
