@@ -35,12 +35,14 @@ def _check_device():
 _DT = {torch.bfloat16: _lib.SLA_BF16, torch.float16: _lib.SLA_FP16, torch.float32: _lib.SLA_FP32}
 
 
+# Addresses and stream handles go to ctypes as plain integers (every pointer argument is declared c_void_p): short
+# calls are bound by this layer, where a c_void_p object a pointer and a Stream object a call cost as much as a launch.
 def _p(t: Optional[torch.Tensor]):
-    return None if t is None else C.c_void_p(t.data_ptr())
+    return None if t is None else t.data_ptr()
 
 
 def _stream(t: torch.Tensor):
-    return C.c_void_p(torch.cuda.current_stream(t.device).cuda_stream)
+    return torch._C._cuda_getCurrentRawStream(t.get_device())
 
 
 def _require_cuda(*ts: torch.Tensor):
@@ -177,7 +179,7 @@ def block_map_pooled(pooled: PooledSums, topk_ratio: float, want_map: bool = Fal
     ci = torch.empty((B, H, mb * max(topk, 0)), dtype=torch.int32, device=dev) if want_cols else None
     ws = _workspace(shape, _lib.OP_BLOCK_MAP, dev)
     check(lib.sla_block_map_pooled(C.byref(shape), _p(pooled.buf), _p(lut), _p(smap), _p(co), _p(ci), _p(ws), ws.numel(),
-                                   torch.cuda.current_stream(dev).cuda_stream))
+                                   _stream(pooled.buf)))
     return BlockMap(lut, topk, nb, smap, co, ci)
 
 
@@ -290,7 +292,7 @@ def prepare_linear(k, v, weight, bias, L_blocks_topk: int, BLKQ=64, BLKK=64, fea
     w, b = weight.detach(), (bias.detach() if bias is not None else None)
     if stream is not None:
         stream.wait_stream(torch.cuda.current_stream(dev))
-        handle = C.c_void_p(stream.cuda_stream)
+        handle = stream.cuda_stream
     else:
         handle = _stream(k)
     check(lib.sla_fwd_prepare(C.byref(shape), _p(k), _p(v), _p(w), _p(b), _p(lin_state), _p(ws), ws.numel(), handle))
@@ -397,7 +399,7 @@ def sage_prepare(q, k, v, weight, bias, topk: int, feature="softmax", sparse_onl
     w, b = weight.detach(), (bias.detach() if bias is not None else None)
     if stream is not None:
         stream.wait_stream(torch.cuda.current_stream(q.device))
-        handle = C.c_void_p(stream.cuda_stream)
+        handle = stream.cuda_stream
     else:
         handle = _stream(q)
     check(lib.sage_sla_prepare(C.byref(shape), _p(q), _p(k), _p(v), _p(w), _p(b), _p(lin_state), _p(ws), ws.numel(),
