@@ -336,8 +336,9 @@ class _SLAFused(torch.autograd.Function):
                               _p(lse), _p(lin_state), _p(ws), ws.numel(), _stream(q)))
         _check_device()
         if need_grad:
-            # the "unselected" scope's backward reads phi(q), phi(k) and the selected blocks' share from the workspace
-            kept = (ws,) if impl_flags & _lib.FLAG_LINEAR_UNSELECTED else ()
+            # the "unselected" scope's backward reads phi(q), phi(k) and the selected blocks' share from the workspace,
+            # unless it is a caller's, who may hand it to another forward before this one's backward
+            kept = (ws,) if impl_flags & _lib.FLAG_LINEAR_UNSELECTED and prep is None else ()
             ctx.save_for_backward(q, k, v, o_s, lse, lin_state, weight, bm.lut, bm.col_offsets, bm.col_index, *kept)
             ctx.sla_shape = shape
             ctx.feature = feature

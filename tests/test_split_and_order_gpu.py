@@ -1,5 +1,6 @@
 """Dispatch edges of the preparation and ordering kernels: each result against another route to the same values."""
 import ctypes as C
+import gc
 import subprocess
 import sys
 
@@ -11,6 +12,14 @@ from oracle import sla_oracle as O
 from sla_b200 import _lib, ops
 
 pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module", autouse=True)
+def _collect_maps_afterwards():
+    """A block map and its 0/1 tensor refer to each other: their memory goes here, not in the middle of a later test
+    that watches the allocator."""
+    yield
+    gc.collect()
 
 
 def _randn(shape, seed, dtype=torch.bfloat16):
@@ -87,6 +96,24 @@ def test_saved_workspace_backward_equals_the_recomputing_one(L, D, BLKQ, feature
     for a, t in zip(out, ts):
         assert torch.equal(a, t.grad)
     assert torch.equal(dw, m.proj_l.weight.grad) and torch.equal(db, m.proj_l.bias.grad)
+
+
+def test_one_preparation_serves_two_forwards_before_their_backwards():
+    L, D = 900, 64
+    m = sla_b200.SparseLinearAttention(D, 0.25, "elu", linear_scope="unselected").cuda()
+    w, b = m.proj_l.weight.detach().normal_(0, 0.05), m.proj_l.bias.detach()
+    k, v, do = (_randn((1, 2, L, D), 30 + i) for i in range(3))
+    qs = [_randn((1, 2, L, D), 40 + i).requires_grad_(True) for i in range(2)]
+    bms = [ops.block_map(q.detach(), k, 0.25, 64, 64, want_cols=True) for q in qs]
+    prep = ops.prepare_linear(k, v, w, b, bms[0].topk, 64, 64, "elu", m.impl_flags)
+    outs = [ops.sla_attention(q, k, v, w, b, bm, 64, 64, "elu", m.impl_flags, prep) for q, bm in zip(qs, bms)]
+    for o in outs:
+        o.backward(do)
+    for q, bm in zip(qs, bms):
+        alone = q.detach().requires_grad_(True)
+        ops.sla_attention(alone, k, v, w, b, bm, 64, 64, "elu", m.impl_flags).backward(do)
+        assert torch.equal(alone.grad, q.grad)
+
 
 
 def test_first_call_of_a_thread_may_be_a_backward():
