@@ -664,112 +664,142 @@ int run_k_mean(const sla_shape* s, const void* k, float* partial, float* kmean, 
 namespace sla {
 // ---- 8. the step before the path: per-head RMS norm and rotary embedding of q and k, with the block sums the mask
 // prediction needs taken from the rows while they are in registers ----
-// One CTA = one block of rows of one head (z = 0: a query block, z = 1: a KV block). A row is spread over D/8
+// One CTA = one block of rows of up to four heads (z = 0: a query block, z = 1: a KV block). A row is spread over D/8
 // threads with 16-byte loads and stores. Per row: y = x * rsqrt(mean(x^2) + eps) * g (skipped when g is NULL), then
 // the rotation of each pair by the row's angles (skipped when cos is NULL): pairs are (y[2i], y[2i+1]) when
 // `interleaved`, else (y[i], y[i + D/2]). The result is rounded to T, stored, and the ROUNDED values are summed per
 // column into sums[bh][block][D] (fp32): the mask prediction then starts from the same bits a separate pooling
 // pass over the stored tensor would read.
+// What bounds it: a row's shuffles, rotation and stores follow its load, and a CTA that did them in turn kept the memory
+// busy half of the time (123 us for 12 heads of 32760 tokens, q and k: 402 MB, 3.3 TB/s). The same rows of up to four
+// heads go through one CTA: the rotation tables, twice the bytes of a row, are then in the L1 from the second head on,
+// and the next head's rows are on their way while this head's are worked on: 112 us. The issue slots are half used
+// then, at three CTAs per SM.
+constexpr int kNormBatch = 4;   // passes in flight
+
 template <typename T, int D>
-__global__ void __launch_bounds__(256) qk_norm_rope_pool_kernel(
+__global__ void __launch_bounds__(256, 3) qk_norm_rope_pool_kernel(
     const T* __restrict__ q_in, const T* __restrict__ k_in, const float* __restrict__ gq, const float* __restrict__ gk,
     const float* __restrict__ cs, const float* __restrict__ sn, float eps, int interleaved, T* __restrict__ q_out,
-    T* __restrict__ k_out, float* __restrict__ qsum, float* __restrict__ ksum, int L, int blkq, int blkk) {
+    T* __restrict__ k_out, float* __restrict__ qsum, float* __restrict__ ksum, int L, int blkq, int blkk, int nbh, int hpc) {
   constexpr int TPR = D / 8;       // threads per row
   constexpr int RP = 256 / TPR;    // rows per pass
   __shared__ float red[RP][D];
+  __shared__ __align__(16) unsigned char ring[2 * kNormBatch * 256 * 16];
   const bool is_k = blockIdx.z == 1;
   const int blk = is_k ? blkk : blkq;
   const int nblk = (L + blk - 1) / blk;
   if (static_cast<int>(blockIdx.x) >= nblk) return;
-  const int bh = blockIdx.y, ib = blockIdx.x;
+  const int ib = blockIdx.x;
   const int tid = threadIdx.x, rg = tid / TPR, c = (tid % TPR) * 8;
   const int row0 = ib * blk, row1 = min(L, row0 + blk);
-  const T* src = (is_k ? k_in : q_in) + static_cast<size_t>(bh) * L * D;
-  T* dst = (is_k ? k_out : q_out) + static_cast<size_t>(bh) * L * D;
   const float* gw = is_k ? gk : gq;
   float g8[8];
 #pragma unroll
   for (int i = 0; i < 8; ++i) g8[i] = gw ? gw[c + i] : 1.f;
-  float acc[8];
-#pragma unroll
-  for (int i = 0; i < 8; ++i) acc[i] = 0.f;
-  // every thread runs the same number of passes (the shuffles below need the whole row group); rows past the
-  // block are computed on zeros and dropped
   const int passes = (blk + RP - 1) / RP;
-  for (int it = 0; it < passes; ++it) {
-    const int r = row0 + it * RP + rg;
-    const bool live = r < row1;
-    float x[8];
-    if (live) {
-      uint4 raw = *reinterpret_cast<const uint4*>(src + static_cast<size_t>(r) * D + c);
-      const uint32_t* w = reinterpret_cast<const uint32_t*>(&raw);
+  const int bh_first = blockIdx.y * hpc, bh_end = min(nbh, bh_first + hpc);
+  // Every thread runs the same number of passes (the shuffles below need the whole row group); rows past the block are
+  // computed on zeros and dropped. kNormBatch passes at a time come through shared memory, every thread its own 16-byte
+  // slots, and the next batch, of this head or the next, is copied while this one is worked on.
+  auto slot = [&](int b, int u) { return ring + (((b & 1) * kNormBatch + u) * 256 + tid) * 16; };
+  auto request = [&](int bh, int it0, int b) {
+    const T* src = (is_k ? k_in : q_in) + static_cast<size_t>(bh) * L * D;
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const float2 f = Elem<T>::unpack2(w[i]);
-        x[2 * i] = f.x; x[2 * i + 1] = f.y;
-      }
-    } else {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) x[i] = 0.f;
+    for (int u = 0; u < kNormBatch; ++u) {
+      const int r = row0 + (it0 + u) * RP + rg;
+      cp_async16(smem_u32(slot(b, u)), src + static_cast<size_t>(min(r, L - 1)) * D + c, r < row1);
     }
-    if (gw != nullptr) {
-      float ss = 0.f;
+  };
+  request(bh_first, 0, 0);
+  cp_async_commit();
+  int batch = 0;
+  for (int bh = bh_first; bh < bh_end; ++bh) {
+    T* dst = (is_k ? k_out : q_out) + static_cast<size_t>(bh) * L * D;
+    float acc[8];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) ss += x[i] * x[i];
+    for (int i = 0; i < 8; ++i) acc[i] = 0.f;
+    for (int it0 = 0; it0 < passes; it0 += kNormBatch, ++batch) {
+      const bool more = it0 + kNormBatch < passes;
+      if (more || bh + 1 < bh_end) request(more ? bh : bh + 1, more ? it0 + kNormBatch : 0, batch + 1);
+      cp_async_commit();
+      cp_async_wait<1>();
 #pragma unroll
-      for (int o = 1; o < TPR; o <<= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-      const float inv = rsqrtf(ss / static_cast<float>(D) + eps);
+      for (int u = 0; u < kNormBatch; ++u) {
+        if (it0 + u >= passes) break;
+        const int r = row0 + (it0 + u) * RP + rg;
+        const bool live = r < row1;
+        float x[8];
+        {
+          const uint4 raw = *reinterpret_cast<const uint4*>(slot(batch, u));
+          const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
 #pragma unroll
-      for (int i = 0; i < 8; ++i) x[i] = x[i] * inv * g8[i];
-    }
-    if (cs != nullptr) {
-      const int rr = live ? r : 0;
-      const float* cr = cs + static_cast<size_t>(rr) * (D / 2);
-      const float* sr = sn + static_cast<size_t>(rr) * (D / 2);
-      if (interleaved) {
-        const float4 c4 = *reinterpret_cast<const float4*>(cr + c / 2), s4 = *reinterpret_cast<const float4*>(sr + c / 2);
-        const float cc[4] = {c4.x, c4.y, c4.z, c4.w}, sv[4] = {s4.x, s4.y, s4.z, s4.w};
+          for (int i = 0; i < 4; ++i) {
+            const float2 f = Elem<T>::unpack2(w[i]);
+            x[2 * i] = f.x; x[2 * i + 1] = f.y;
+          }
+        }
+        if (gw != nullptr) {
+          float ss = 0.f;
+#pragma unroll
+          for (int i = 0; i < 8; ++i) ss += x[i] * x[i];
+#pragma unroll
+          for (int o = 1; o < TPR; o <<= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+          const float inv = rsqrtf(ss / static_cast<float>(D) + eps);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) x[i] = x[i] * inv * g8[i];
+        }
+        if (cs != nullptr) {
+          if (interleaved) {
+            const size_t to = static_cast<size_t>(live ? r : 0) * (D / 2) + c / 2;
+            const float4 c4 = __ldg(reinterpret_cast<const float4*>(cs + to)), s4 = __ldg(reinterpret_cast<const float4*>(sn + to));
+            const float cc[4] = {c4.x, c4.y, c4.z, c4.w}, sv[4] = {s4.x, s4.y, s4.z, s4.w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const float a = x[2 * i], b = x[2 * i + 1];
+              x[2 * i] = a * cc[i] - b * sv[i];
+              x[2 * i + 1] = a * sv[i] + b * cc[i];
+            }
+          } else {
+            // the partner of column j is column j +- D/2, held by the lane TPR/2 away in the same row group
+            const int rr = live ? r : 0;
+            const float* cr = cs + static_cast<size_t>(rr) * (D / 2);
+            const float* sr = sn + static_cast<size_t>(rr) * (D / 2);
+            const bool upper = c >= D / 2;
+            const int j0 = upper ? c - D / 2 : c;
+            const float4 ca = *reinterpret_cast<const float4*>(cr + j0), cb = *reinterpret_cast<const float4*>(cr + j0 + 4);
+            const float4 sa = *reinterpret_cast<const float4*>(sr + j0), sb = *reinterpret_cast<const float4*>(sr + j0 + 4);
+            const float cc[8] = {ca.x, ca.y, ca.z, ca.w, cb.x, cb.y, cb.z, cb.w};
+            const float sv[8] = {sa.x, sa.y, sa.z, sa.w, sb.x, sb.y, sb.z, sb.w};
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              const float other = __shfl_xor_sync(0xffffffffu, x[i], TPR / 2);
+              x[i] = upper ? x[i] * cc[i] + other * sv[i] : x[i] * cc[i] - other * sv[i];
+            }
+          }
+        }
+        uint4 outv;
+        uint32_t* ow = reinterpret_cast<uint32_t*>(&outv);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          const float a = x[2 * i], b = x[2 * i + 1];
-          x[2 * i] = a * cc[i] - b * sv[i];
-          x[2 * i + 1] = a * sv[i] + b * cc[i];
+          ow[i] = Elem<T>::pack2(x[2 * i], x[2 * i + 1]);
+          const float2 f = Elem<T>::unpack2(ow[i]);
+          if (live) { acc[2 * i] += f.x; acc[2 * i + 1] += f.y; }
         }
-      } else {
-        // the partner of column j is column j +- D/2, held by the lane TPR/2 away in the same row group
-        const bool upper = c >= D / 2;
-        const int j0 = upper ? c - D / 2 : c;
-        const float4 ca = *reinterpret_cast<const float4*>(cr + j0), cb = *reinterpret_cast<const float4*>(cr + j0 + 4);
-        const float4 sa = *reinterpret_cast<const float4*>(sr + j0), sb = *reinterpret_cast<const float4*>(sr + j0 + 4);
-        const float cc[8] = {ca.x, ca.y, ca.z, ca.w, cb.x, cb.y, cb.z, cb.w};
-        const float sv[8] = {sa.x, sa.y, sa.z, sa.w, sb.x, sb.y, sb.z, sb.w};
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const float other = __shfl_xor_sync(0xffffffffu, x[i], TPR / 2);
-          x[i] = upper ? x[i] * cc[i] + other * sv[i] : x[i] * cc[i] - other * sv[i];
-        }
+        if (live) *reinterpret_cast<uint4*>(dst + static_cast<size_t>(r) * D + c) = outv;
       }
     }
-    uint4 outv;
-    uint32_t* ow = reinterpret_cast<uint32_t*>(&outv);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      ow[i] = Elem<T>::pack2(x[2 * i], x[2 * i + 1]);
-      const float2 f = Elem<T>::unpack2(ow[i]);
-      if (live) { acc[2 * i] += f.x; acc[2 * i + 1] += f.y; }
-    }
-    if (live) *reinterpret_cast<uint4*>(dst + static_cast<size_t>(r) * D + c) = outv;
-  }
-#pragma unroll
-  for (int i = 0; i < 8; ++i) red[rg][c + i] = acc[i];
-  __syncthreads();
-  if (tid < D) {
-    float sm = 0.f;
+    for (int i = 0; i < 8; ++i) red[rg][c + i] = acc[i];
+    __syncthreads();
+    if (tid < D) {
+      float sm = 0.f;
 #pragma unroll 4
-    for (int g = 0; g < RP; ++g) sm += red[g][tid];
-    float* out = (is_k ? ksum : qsum) + (static_cast<size_t>(bh) * nblk + ib) * D;
-    out[tid] = sm;
+      for (int g = 0; g < RP; ++g) sm += red[g][tid];
+      float* out = (is_k ? ksum : qsum) + (static_cast<size_t>(bh) * nblk + ib) * D;
+      out[tid] = sm;
+    }
+    __syncthreads();     // the sums of the next head overwrite the slots
   }
 }
 
@@ -777,8 +807,8 @@ __global__ void __launch_bounds__(256) qk_norm_rope_pool_kernel(
 // pooled_k = round_T(ksum / nx - kmean). The last line is where this path departs from utils.py:56 + :40, which
 // round every element of k - mean(k) to T before pooling: the block mean of those rounding errors (well below one
 // unit in the last place of the pooled value) is not reproduced.
-// One CTA per head, 1024 threads = 8 groups of 128 columns: group g sums the blocks j = g (mod 8) with four loads in
-// flight, the eight partial sums are added in a fixed order.
+// One CTA per head, 1024 threads = 8 groups of 128 columns: group g sums the blocks j = g (mod 8) in four chains,
+// sixteen loads in flight, the eight partial sums are added in a fixed order.
 template <typename TIn>
 __global__ void __launch_bounds__(1024) pooled_kmean_kernel(const float* __restrict__ ksum, float* __restrict__ kmean,
                                                             int L, int nb, int D) {
@@ -788,6 +818,7 @@ __global__ void __launch_bounds__(1024) pooled_kmean_kernel(const float* __restr
   float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
   if (d < D) {
     int j = g;
+#pragma unroll 4
     for (; j + 24 < nb; j += 32) {
       s0 += base[static_cast<size_t>(j) * D + d];
       s1 += base[static_cast<size_t>(j + 8) * D + d];
@@ -834,9 +865,11 @@ static int qk_prepare_typed(const sla_shape* s, const T* q_in, const T* k_in, co
   const int bh = s->B * s->H, mb = ceil_div(s->L, s->BLKQ), nb = ceil_div(s->L, s->BLKK);
   float* qsum = reinterpret_cast<float*>(sums);
   float* ksum = reinterpret_cast<float*>(sums + ws_round(size_t(bh) * mb * s->D * 4));
-  qk_norm_rope_pool_kernel<T, D><<<dim3(max(mb, nb), bh, 2), 256, 0, st>>>(q_in, k_in, gq, gk, cs, sn, eps, interleaved,
-                                                                            q_out, k_out, qsum, ksum, s->L, s->BLKQ,
-                                                                            s->BLKK);
+  // heads per CTA: four once that still leaves several CTAs for every resident slot (148 SMs of eight)
+  const long long ctas = 2LL * max(mb, nb) * bh;
+  const int hpc = ctas >= 8192 ? 4 : (ctas >= 4096 ? 2 : 1);
+  qk_norm_rope_pool_kernel<T, D><<<dim3(max(mb, nb), ceil_div(bh, hpc), 2), 256, 0, st>>>(
+      q_in, k_in, gq, gk, cs, sn, eps, interleaved, q_out, k_out, qsum, ksum, s->L, s->BLKQ, s->BLKK, bh, hpc);
   SLA_LAUNCH_OK();
   return SLA_OK;
 }
