@@ -43,7 +43,7 @@ void count_launch();
 // launch_pdl<false> is an ordinary launch through the same interface. The forward path uses it: there the linear-branch
 // state runs on a second stream next to the mask prediction, and a kernel that becomes resident early and sits in
 // pdl_wait() holds SM slots the other stream's kernels could use; no gain was measured there. The backward is one
-// chain of eight kernels on one stream and launches programmatically (about 1 % of the step at L = 32760 with 12
+// chain of six kernels on one stream and launches programmatically (about 1 % of the step at L = 32760 with 12
 // heads, 5-8 % with one or two heads per GPU).
 template <bool Programmatic = true, typename... KArgs, typename... Args>
 inline cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
