@@ -35,6 +35,17 @@ inline WsBlockMap ws_block_map(const sla_shape* s) {
   return w;
 }
 
+// The split of a head's rows into chunks fixes the order of the fp32 sums. It depends on L alone, never on B or H, so a
+// (batch, head) unit gives the same bits whatever else is in the batch and however the units are sharded over GPUs.
+// At most 64 chunks. Up to 4096 rows they have 256, since short calls have too few CTAs (8 heads of 4096 rows: backward
+// row pass 43 -> 28 us); above, 512, since the partials then cost more than the wider split gives (layer call of 32
+// heads of 6165 rows: 321 us with 512, 332 with 256).
+inline int ws_row_chunks(int L) {
+  const int fine = ws_ceil_div(L, 256), coarse = ws_ceil_div(L, 512);
+  const int n = L <= 4096 ? fine : (coarse > 16 ? coarse : 16);
+  return n > 64 ? 64 : n;
+}
+
 // ---- linear-branch state: partial H (D x D) and z (D) per chunk of rows, fp32 ----
 struct WsLinearState {
   size_t partial;  // fp32 [BH][NCH][D*D + D]
@@ -45,11 +56,7 @@ struct WsLinearState {
 inline WsLinearState ws_linear_state(const sla_shape* s) {
   WsLinearState w;
   size_t bh = size_t(s->B) * s->H;
-  // The split of a head's rows into chunks fixes the order of the fp32 sums. It depends on L alone, never on
-  // B or H, so a (batch, head) unit gives the same bits whatever else is in the batch and however the units are
-  // sharded over GPUs: at most 64 chunks per head, at least 256 rows per chunk.
-  int nch = ws_ceil_div(s->L, 256);
-  if (nch > 64) nch = 64;
+  int nch = ws_row_chunks(s->L);
   int rows = (ws_ceil_div(s->L, nch) + 127) / 128 * 128;
   w.rows = rows;
   w.nch = ws_ceil_div(s->L, rows);
@@ -96,9 +103,8 @@ struct WsBwd {
 inline WsBwd ws_bwd(const sla_shape* s) {
   WsBwd w;
   size_t bh = size_t(s->B) * s->H;
-  // chunks of the linear backward's row passes: a function of L alone, like ws_linear_state
-  int nch = ws_ceil_div(s->L, 256);
-  if (nch > 64) nch = 64;
+  // chunks of the linear backward's row passes: as in ws_linear_state
+  int nch = ws_row_chunks(s->L);
   int rows = (ws_ceil_div(s->L, nch) + 127) / 128 * 128;
   w.rows = rows;
   w.nch = ws_ceil_div(s->L, rows);
