@@ -206,14 +206,16 @@ __device__ inline uint32_t smem_u32(const void* p) {
 }
 
 // 16-byte async copy global -> shared; `valid == false` writes zeros instead of reading.
+// The "memory" clobbers keep plain loads of the copied bytes behind the wait and in front of the next copy into the same
+// place: the rings of which every thread reads its own slots back have no barrier there that would do it.
 __device__ inline void cp_async16(uint32_t saddr, const void* gptr, bool valid) {
   int sz = valid ? 16 : 0;
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(saddr), "l"(gptr), "r"(sz));
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(saddr), "l"(gptr), "r"(sz) : "memory");
 }
-__device__ inline void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
+__device__ inline void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N>
 __device__ inline void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;\n" ::"n"(N));
+  asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 
 // ---------------------------------------------------------------------------------------------
