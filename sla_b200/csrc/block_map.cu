@@ -57,15 +57,29 @@ __global__ void __launch_bounds__(256) colsum_kernel(const TIn* __restrict__ k, 
 }
 
 // ---- 2. mean[bh][d] = round_T(sum / L) (torch.mean keeps the input dtype, utils.py:56) ----
+// kMeanBatch loads are in flight, the sum is taken in order. What is left behind the full batches is a guarded batch, not a
+// loop of its own whose loads would come one after another (8 heads, K of 15 chunks: 5.3 us with such a loop, 2.2 so).
+constexpr int kMeanBatch = 16;
+
 template <typename TIn>
 __global__ void kmean_finalize_kernel(const float* __restrict__ partial, float* __restrict__ kmean, int L,
                                       int nch, int D) {
   pdl_wait();
   int bh = blockIdx.x, d = threadIdx.x;
   if (d >= D) return;
+  const float* p = partial + static_cast<size_t>(bh) * nch * D + d;
   float s = 0.f;
-#pragma unroll 16
-  for (int c = 0; c < nch; ++c) s += partial[(static_cast<size_t>(bh) * nch + c) * D + d];   // loads batched, sum in order
+  int c = 0;
+  for (; c + kMeanBatch <= nch; c += kMeanBatch) {
+#pragma unroll
+    for (int u = 0; u < kMeanBatch; ++u) s += p[static_cast<size_t>(c + u) * D];
+  }
+  float x[kMeanBatch];
+#pragma unroll
+  for (int u = 0; u < kMeanBatch; ++u) x[u] = c + u < nch ? p[static_cast<size_t>(c + u) * D] : 0.f;
+#pragma unroll
+  for (int u = 0; u < kMeanBatch; ++u)
+    if (c + u < nch) s += x[u];
   kmean[static_cast<size_t>(bh) * D + d] = round_to<TIn>(s / static_cast<float>(L));
 }
 
