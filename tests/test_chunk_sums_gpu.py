@@ -3,8 +3,9 @@ kernels change."""
 import pytest
 import torch
 
+import sla_b200
 from oracle import sla_oracle as O
-from sla_b200 import ops
+from sla_b200 import _lib, ops
 
 pytestmark = pytest.mark.gpu
 
@@ -48,3 +49,23 @@ def test_mean_of_an_unfilled_batch_takes_no_longer():
     full, short = run(8192), run(7680)
     print(f"kmean_finalize: 15 chunks {short:.2f} us, 16 chunks {full:.2f} us")
     assert short < 1.4 * full, (short, full)
+
+
+def _launches(fn):
+    before = _lib.lib.sla_launch_count()
+    out = fn()
+    return _lib.lib.sla_launch_count() - before, out
+
+
+# 64 blocks of 8 chunks a unit: the line lies at 16 units
+@pytest.mark.parametrize("D,units", [(64, 17), (128, 24)])
+def test_many_units_do_not_repeat_the_maxima_of_v(D, units):
+    """Above the line V's scales come from a kernel of their own, with the same bits as where every block makes them."""
+    q, k, v = (_randn((1, units, 4096, D), 30 + i) for i in range(3))
+    m = sla_b200.SageSparseLinearAttention(D, 0.1).cuda()
+    m.overlap_prepare = False
+    with torch.no_grad():
+        n_all, out = _launches(lambda: m(q, k, v))
+        n_few, few = _launches(lambda: m(*(t[:, :16].contiguous() for t in (q, k, v))))
+    assert n_all == n_few + 1
+    assert torch.equal(out[:, :16], few)
