@@ -125,14 +125,15 @@ int sla_fwd_prepare(const sla_shape* s, const void* k, const void* v, const floa
   if (!all_aligned({k, v, lin_state, ws})) return SLA_ERR_BAD_ALIGN;
   if (s->flags & SLA_FLAG_SPARSE_ONLY) return SLA_ERR_UNSUPPORTED;
   WsLinearState wl = ws_linear_state(s);
-  if (ws_bytes < ws_fwd_total(s)) return SLA_ERR_WS_TOO_SMALL;
+  const WsFwd wf = ws_fwd(s);
+  if (ws_bytes < wf.total) return SLA_ERR_WS_TOO_SMALL;
   unsigned char* base = static_cast<unsigned char*>(ws);
-  void* wbits = base + wl.total;
+  void* wbits = base + wf.wbits;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   ProjConvert proj;
   rc = start_convert_proj(s, w, bias, wbits, &proj, st);
   if (rc != SLA_OK) return rc;
-  rc = run_linear_state(s, k, v, lin_state, reinterpret_cast<float*>(base + wl.partial), wl.nch, wl.rows, st, proj);
+  rc = run_linear_state(s, k, v, lin_state, reinterpret_cast<float*>(base + wf.partial), wl.nch, wl.rows, st, proj);
   if (rc != SLA_OK) return rc;
   return run_state_proj(s, lin_state, wbits, st);
 }
@@ -165,16 +166,17 @@ static int fwd_impl(const sla_shape* s, const void* q, const void* k, const void
   }
   if (!w || !lin_state || !ws) return SLA_ERR_NULL;
   WsLinearState wl = ws_linear_state(s);
-  if (ws_bytes < ws_fwd_total(s)) return SLA_ERR_WS_TOO_SMALL;
+  const WsFwd wf = ws_fwd(s);
+  if (ws_bytes < wf.total) return SLA_ERR_WS_TOO_SMALL;
   unsigned char* base = static_cast<unsigned char*>(ws);
-  void* wbits = base + wl.total;
+  void* wbits = base + wf.wbits;
   const bool unselected = (s->flags & SLA_FLAG_LINEAR_UNSELECTED) != 0;
   if (unselected && legacy) return SLA_ERR_UNSUPPORTED;
   if (!(s->flags & SLA_FLAG_STATE_READY)) {
     ProjConvert proj;
     rc = start_convert_proj(s, w, bias, wbits, &proj, st);
     if (rc != SLA_OK) return rc;
-    rc = run_linear_state(s, k, v, lin_state, reinterpret_cast<float*>(base + wl.partial), wl.nch, wl.rows, st, proj);
+    rc = run_linear_state(s, k, v, lin_state, reinterpret_cast<float*>(base + wf.partial), wl.nch, wl.rows, st, proj);
     if (rc != SLA_OK) return rc;
     rc = run_state_proj(s, lin_state, wbits, st);
     if (rc != SLA_OK) return rc;
@@ -183,7 +185,7 @@ static int fwd_impl(const sla_shape* s, const void* q, const void* k, const void
   if (unselected) {
     // sparse branch; then the same block lists once more without softmax on (phi(q), phi(k), v) for the
     // selected blocks' share of the linear state, which the read-out takes off the all-token state
-    unsigned char* ub = base + wl.total + ws_fwd_extra(s);
+    unsigned char* ub = base + wf.unsel;
     WsUnselected wu = ws_unselected(s);
     void* os_buf = o_s ? o_s : o;
     FwdParams ps = make_fwd(s, q, k, v, lut, os_buf, nullptr, lse, nullptr, nullptr);
@@ -459,8 +461,7 @@ int sla_bwd_saved(const sla_shape* s, const void* q, const void* k, const void* 
   if (fwd_ws_bytes < ws_fwd_total(s)) return SLA_ERR_WS_TOO_SMALL;
   sla_shape saved = *s;
   saved.flags |= SLA_FLAG_FWD_SAVED;
-  const unsigned char* fwd_ub =
-      static_cast<const unsigned char*>(fwd_ws) + ws_linear_state(s).total + ws_fwd_extra(s);
+  const unsigned char* fwd_ub = static_cast<const unsigned char*>(fwd_ws) + ws_fwd(s).unsel;
   return bwd_impl(&saved, q, k, v, o_s, lse, d_o, lut, col_offsets, col_index, w, lin_state, dq, dk, dv, dw, dbias, ws,
                   ws_bytes, fwd_ub, stream);
 }

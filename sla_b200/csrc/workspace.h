@@ -83,11 +83,30 @@ inline WsUnselected ws_unselected(const sla_shape* s) {
   w.total = o;
   return w;
 }
-inline size_t ws_fwd_total(const sla_shape* s) {
-  size_t t = ws_linear_state(s).total + ws_fwd_extra(s);
-  if (s->flags & SLA_FLAG_LINEAR_UNSELECTED) t += ws_unselected(s).total;
-  return t;
+// ---- forward. In the "unselected" scope the workspace may be kept until the backward: the chunk partials, which nothing
+// reads once the state is reduced, lie where phi(q), phi(k), C_num are written after that. ----
+struct WsFwd {
+  size_t partial;  // WsLinearState
+  size_t wbits;    // ws_fwd_extra
+  size_t unsel;    // WsUnselected
+  size_t total;
+};
+inline WsFwd ws_fwd(const sla_shape* s) {
+  WsFwd w;
+  const size_t lin = ws_linear_state(s).total, proj = ws_fwd_extra(s);
+  if (s->flags & SLA_FLAG_LINEAR_UNSELECTED) {
+    const size_t u = ws_unselected(s).total;
+    w.wbits = 0;
+    w.partial = w.unsel = proj;
+    w.total = proj + (u > lin ? u : lin);
+  } else {
+    w.partial = 0;
+    w.wbits = lin;
+    w.unsel = w.total = lin + proj;
+  }
+  return w;
 }
+inline size_t ws_fwd_total(const sla_shape* s) { return ws_fwd(s).total; }
 
 // ---- backward ----
 struct WsBwd {
