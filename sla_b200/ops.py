@@ -304,7 +304,7 @@ class _SLAFused(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, q, k, v, weight, bias, bm: BlockMap, BLKQ, BLKK, feature, need_grad, impl_flags, prep,
-                out=None, gather_ptrs=None):
+                out=None, gather_ptrs=None, keep_intermediates=True):
         B, H, L, D = q.shape
         shape = make_shape(B, H, L, D, BLKQ, BLKK, bm.topk, q.dtype, feature, flags=impl_flags)
         dev = q.device
@@ -338,7 +338,7 @@ class _SLAFused(torch.autograd.Function):
         if need_grad:
             # the "unselected" scope's backward reads phi(q), phi(k) and the selected blocks' share from the workspace,
             # unless it is a caller's, who may hand it to another forward before this one's backward
-            kept = (ws,) if impl_flags & _lib.FLAG_LINEAR_UNSELECTED and prep is None else ()
+            kept = (ws,) if impl_flags & _lib.FLAG_LINEAR_UNSELECTED and prep is None and keep_intermediates else ()
             ctx.save_for_backward(q, k, v, o_s, lse, lin_state, weight, bm.lut, bm.col_offsets, bm.col_index, *kept)
             ctx.sla_shape = shape
             ctx.feature = feature
@@ -365,24 +365,26 @@ class _SLAFused(torch.autograd.Function):
         else:
             check(lib.sla_bwd(*args, _p(ws), ws.numel(), _stream(q)))
         _check_device()
-        return dq, dk, dv, dw, (db if ctx.has_bias else None), None, None, None, None, None, None, None, None, None
+        return dq, dk, dv, dw, (db if ctx.has_bias else None), *(None,) * 10
 
 
 def sla_attention(q, k, v, weight, bias, bm: BlockMap, BLKQ=64, BLKK=64, feature="softmax",
                   impl_flags: int = 0, prep: Optional[LinearPrep] = None, out: Optional[torch.Tensor] = None,
-                  gather_ptrs=None):
+                  gather_ptrs=None, keep_intermediates: bool = True):
     """o = o_s + proj_l(o_l) for q, k, v already in the 16-bit compute dtype. `prep`: the result of
     `prepare_linear` on the same k, v, weight, bias (already joined into the current stream). `out`: write the
     result there instead of into a new tensor. `gather_ptrs`: up to 8 device addresses (this process's view) of
     further (B, H, L, D) blocks the kernel's epilogue also writes the result to, e.g. this rank's place in every peer
-    GPU's full-size output (`sharding.GatheredOutput`)."""
+    GPU's full-size output (`sharding.GatheredOutput`). `keep_intermediates`: scope "unselected" only; hold phi(q),
+    phi(k) and the selected blocks' share of the linear branch (three times q) for the backward, or let it make them
+    again."""
     _require_cuda(q, k, v, weight)
     need_grad = torch.is_grad_enabled() and any(
         t is not None and t.requires_grad for t in (q, k, v, weight, bias))
     if need_grad and bm.col_offsets is None:
         raise RuntimeError("the block map was built without column lists (want_cols=True) but a backward is needed")
     return _SLAFused.apply(q, k, v, weight, bias, bm, BLKQ, BLKK, feature, need_grad, impl_flags, prep, out,
-                           gather_ptrs)
+                           gather_ptrs, keep_intermediates)
 
 
 def sage_prepare(q, k, v, weight, bias, topk: int, feature="softmax", sparse_only: bool = False,

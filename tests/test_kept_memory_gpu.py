@@ -3,6 +3,7 @@ import pytest
 import torch
 
 import sla_b200
+from sla_b200 import _lib
 
 pytestmark = pytest.mark.gpu
 
@@ -30,3 +31,29 @@ def test_kept_buffer_is_three_times_q(L, D):
     kept = _kept(_module(D)(q, k, v))
     rows = q.numel() // D
     assert [t.numel() for t in kept] and sum(t.numel() for t in kept) <= rows * (3 * 2 * D + 4) + 2 * D * (D + 1) + 6 * 256
+
+
+def _launches_of_backward(m, ts):
+    o = m(*ts)
+    kept = len(_kept(o))
+    before = _lib.lib.sla_launch_count()
+    o.backward(torch.ones_like(o))
+    return kept, _lib.lib.sla_launch_count() - before
+
+
+def test_the_caller_chooses_between_memory_and_recomputation():
+    """Without the kept buffer the backward has two launches more, the feature maps and the product over the selected
+    blocks, and the same gradients."""
+    m = _module(128)
+    grads, seen = [], []
+    for keep in (True, False):
+        m.keep_linear_intermediates = keep
+        m.zero_grad()
+        ts = _inputs(1, 2, 900, 128)
+        seen.append(_launches_of_backward(m, ts))
+        grads.append([t.grad for t in (*ts, m.proj_l.weight, m.proj_l.bias)])
+    (kept, launches), (kept_not, launches_more) = seen
+    assert (kept, kept_not) == (1, 0)
+    assert launches_more == launches + 2
+    for a, b in zip(*grads):
+        assert torch.equal(a, b)
