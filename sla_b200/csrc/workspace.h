@@ -37,9 +37,17 @@ inline WsBlockMap ws_block_map(const sla_shape* s) {
 
 // The split of a head's rows into chunks fixes the order of the fp32 sums. It depends on L alone, never on B or H, so a
 // (batch, head) unit gives the same bits whatever else is in the batch and however the units are sharded over GPUs.
-// At most 64 chunks. Up to 4096 rows they have 256, since short calls have too few CTAs (8 heads of 4096 rows: backward
-// row pass 43 -> 28 us); above, 512, since the partials then cost more than the wider split gives (layer call of 32
-// heads of 6165 rows: 321 us with 512, 332 with 256).
+// Chunks are whole tiles of 128 rows: 256 rows up to L = 4096; above, about a sixteenth of the rows but no less than that
+// of 512-row chunks (384 rows to L = 6144, 512 to 32768), at most 64 chunks.
+// The rule cannot look at how many units there are, and they decide what pays: few leave SMs without a chunk, many pay for
+// the partials of a finer split (66 KB a chunk at head dim 128). Device time with 512 rows everywhere against this rule,
+// head dim 128, module forward | training step, top-k 0.2:
+//   units   L = 1024             2048                 4096                    4097
+//     2   56 / 50 | 140 / 122    60 / 54 | 154 / 133    70 / 65 | 189 / 167      73 / 73 | 193 / 185 us
+//     8   56 / 51 | 143 / 125    62 / 56 | 162 / 140    77 / 72 | 256 / 235      81 / 78 | 260 / 253
+//    32   62 / 58 | 193 / 176    97 / 99 | 321 / 308   181 / 190 | 643 / 662    191 / 190 | 704 / 719
+//    72   94 / 97 | 290 / 287   156 / 165 | 547 / 557  357 / 375 | 1373 / 1414  384 / 392 | 1479 / 1474
+// At head dim 64, a quarter of the bytes a chunk, the finer split never lost more than 2.5 %.
 inline int ws_row_chunks(int L) {
   const int fine = ws_ceil_div(L, 256), coarse = ws_ceil_div(L, 512);
   const int n = L <= 4096 ? fine : (coarse > 16 ? coarse : 16);
