@@ -879,7 +879,9 @@ static int qk_prepare_typed(const sla_shape* s, const T* q_in, const T* k_in, co
   const int bh = s->B * s->H, mb = ceil_div(s->L, s->BLKQ), nb = ceil_div(s->L, s->BLKK);
   float* qsum = reinterpret_cast<float*>(sums);
   float* ksum = reinterpret_cast<float*>(sums + ws_round(size_t(bh) * mb * s->D * 4));
-  // heads per CTA: four once that still leaves several CTAs for every resident slot (148 SMs of eight)
+  // Heads per CTA: two, then four, as soon as that is no slower (three CTAs an SM, 444 slots). Head dim 128, 64-row blocks,
+  // one | two | four heads a CTA: 2048 CTAs of one head 30.5 | 30.7 | 34.8 us, 4096 49.3 | 47.2 | 50.2, 6144 69.1 | 64.5 |
+  // 65.6, 8192 92.2 | 87.6 | 86.0, 12288 131.9 | 122.9 | 120.3; head dim 64: 4096 34.8 | 32.8 | 32.8, 12288 88.2 | 78.2 | 73.8.
   const long long ctas = 2LL * max(mb, nb) * bh;
   const int hpc = ctas >= 8192 ? 4 : (ctas >= 4096 ? 2 : 1);
   qk_norm_rope_pool_kernel<T, D><<<dim3(max(mb, nb), ceil_div(bh, hpc), 2), 256, 0, st>>>(
@@ -985,7 +987,7 @@ extern "C" int sla_index_convert(const void* src, int src_bits, void* dst, int d
   int rc = check_device_arch();
   if (rc != SLA_OK) return rc;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const unsigned grid = static_cast<unsigned>(count / 1024 + 1 < 148u * 8u ? count / 1024 + 1 : 148u * 8u);
+  const unsigned grid = static_cast<unsigned>(count / 1024 + 1 < kSms * 8u ? count / 1024 + 1 : kSms * 8u);
   if (src_bits == 32 && dst_bits == 16)
     index_convert_kernel<int32_t, uint16_t><<<grid, 256, 0, st>>>(static_cast<const int32_t*>(src),
                                                                   static_cast<uint16_t*>(dst), count);

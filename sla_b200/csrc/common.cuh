@@ -67,6 +67,8 @@ __device__ __forceinline__ void pdl_entry() { pdl_wait(); pdl_launch_dependents(
 // kernel: some loads from the L2 a thread against a launch of 4-5 us of host time.
 constexpr int kInlineMeanChunks = 8;
 
+constexpr int kSms = 148;      // of a B200
+
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 inline size_t round256(size_t x) { return (x + 255) & ~size_t(255); }
 inline int ceil_div(int a, int b) { return (a + b - 1) / b; }

@@ -169,7 +169,8 @@ __global__ void __launch_bounds__(D / 16 * 32) linear_bwd_q_kernel(LinBwdParams 
 }
 
 // ---------------------------------------------------------------------------------------------
-// Per-head reductions. (1) sum the chunk partials (and, in a CTA of its own, the dK/dV kernel's tile order); (2) G -> dH (T), and the head's dW; dz, db copied.
+// Per-head reductions. (1) sum the chunk partials (and, in CTAs of their own, the dK/dV kernel's tile order and the 16-bit
+// proj_l); (2) G -> dH (T), and the head's dW; dz, db copied.
 // ---------------------------------------------------------------------------------------------
 static_assert(kOrderThreads == 256, "the reduction kernel's block size");
 template <typename T>

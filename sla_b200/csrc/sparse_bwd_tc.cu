@@ -343,7 +343,7 @@ sparse_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_co
     const uint32_t lane_addr = static_cast<uint32_t>((warp & 3) * 32) << 16;
     const int half = row >> 6;
     const float sc = p.scale_log2;
-    const bool key_ok = unit[0] * 128 + row < L;                           // keys past the end give P = 0 (kernel.py:216)
+    const bool key_ok = unit[0] * 128 + row < L;     // keys past the end give P = 0 (kernel.py:216)
     bool ok = !*abortp;
     // A pair meets a buffer again after lcm(2, NB) entries, the other pair having used it in between; the scores are
     // computed in order, so when a pair waits for entry j's it knows that those of entry j - NB are there, and the
@@ -454,7 +454,7 @@ sparse_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_co
             else x[c] = x[c] > 0.f ? x[c] + 1.f : __expf(x[c]);      // elu(x) + 1
           }
         }
-        const bool key_live = unit[0] * 128 + row < L;                        // rows past the end: K was zero-filled, phi must be 0
+        const bool key_live = unit[0] * 128 + row < L;   // rows past the end: K was zero-filled, phi must be 0
         uint32_t phi[CW / 2];                                  // phi(k) rounded to T (core.py:91)
 #pragma unroll
         for (int c = 0; c < CW; c += 2) phi[c >> 1] = key_live ? Elem<T>::pack2(x[c], x[c + 1]) : 0u;

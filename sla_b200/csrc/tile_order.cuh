@@ -1,12 +1,12 @@
 // The order in which the dK/dV kernel's last CTAs take their 128-key tiles: longest list first.
 //
 // A key tile's work is the length of its column lists, and popular KV blocks are selected several times as often as
-// the average (32760 tokens of a (21, 30, 52) latent grid, top-k 25 of 512: mean 34 entries a tile, largest 128). In
-// sequence order such a tile may start last and run alone. The tiles of the last heads are therefore taken largest
-// first. List scheduling on 148 SMs, in units of entries: the busiest SM gets 143 instead of 198 with 2 heads (137 is
-// the mean over the SMs), 827 instead of 884 with 12. Only the last heads: the CTAs in flight share the Q and dO rows
-// of their heads in the L2, and with every tile ordered (groups of 64 MB of rows) a uniform mask of 32 heads, where
-// there is nothing to gain, ran 4 % slower.
+// the average (32760 tokens of a (21, 30, 52) latent grid, top-k 25 of 512: a tile's two lists merge to 34 entries in the
+// mean, to 110-150 for the longest). In sequence order such a tile may start last and run alone. The tiles of the last
+// heads are therefore taken longest first. List scheduling on 148 SMs, counting entries alone: the busiest SM gets 130
+// instead of 174 with 2 heads (119 is the mean over the SMs), 696 instead of 783 with 12 (691). Measured, with 2 heads:
+// dK/dV 271 -> 195 us. Only the last heads: the CTAs in flight share the Q and dO rows of their heads in the L2, and with
+// every tile ordered (groups of 64 MB of rows) a uniform mask of 32 heads, where there is nothing to gain, ran 4 % slower.
 #pragma once
 #include "common.cuh"
 
@@ -28,7 +28,7 @@ inline int order_heads(int ntiles, int D, int bh) {      // last heads with at m
 inline TileOrder make_tile_order(const int32_t* col_offsets, int32_t* order, int nb, int mb, int D, int bh) {
   TileOrder o;
   o.nb = nb; o.ntiles = ceil_div(nb, 2); o.bh = bh;
-  if (static_cast<long long>(o.ntiles) * bh <= 148) return o;
+  if (static_cast<long long>(o.ntiles) * bh <= kSms) return o;
   o.col_offsets = col_offsets; o.order = order;
   o.h0 = bh - order_heads(o.ntiles, D, bh);
   while ((2LL * mb >> o.shift) >= kOrderBins) ++o.shift;   // a tile's two lists hold at most 2 * mb entries
