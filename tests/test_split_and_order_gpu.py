@@ -53,6 +53,8 @@ def test_block_map_at_the_inline_mean_edge(L, dtype):
 @pytest.mark.parametrize("L,D,BLKQ,heads", [(1000, 64, 64, 24), (2500, 128, 128, 9), (19000, 64, 128, 3)])
 def test_tile_order_leaves_the_gradients_alone(L, D, BLKQ, heads):
     """All heads in one call take the ordered tiles (more than one per SM), a head by itself the sequence order."""
+    # At L = 19000 a single head has 149 tiles and an order of its own. Here every head is ordered; the calls whose first
+    # heads are not are in test_tile_order_of_the_last_heads.
     q, k, v, do = (_randn((1, heads, L, D), 10 + i) for i in range(4))
     k[:, :, : L // 3] *= 3                                # popular and unpopular blocks
 
@@ -129,3 +131,38 @@ torch.cuda.synchronize()
 """
     r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stderr[-2000:]
+
+
+def _first_ordered_head(L, D, heads):
+    """order_heads of the library: the last heads with at most 64 MB of 16-bit Q and dO rows."""
+    tiles = ((L + 63) // 64 + 1) // 2
+    assert tiles <= 148 < tiles * heads          # a head by itself takes the sequence order, all of them do not
+    return heads - min(heads, max(1, 1024 * 128 // D // tiles))
+
+
+@pytest.mark.parametrize("scope", ["sparse", "all", "unselected"])
+@pytest.mark.parametrize("L,D,BLKQ,heads", [(16384, 128, 64, 10), (18944, 64, 128, 15), (16300, 128, 128, 9)])
+def test_tile_order_of_the_last_heads(L, D, BLKQ, heads, scope):
+    """The first heads run in sequence and the last ones by length; a head by itself always in sequence."""
+    assert 0 < _first_ordered_head(L, D, heads) < heads
+    q, k, v, do = (_randn((1, heads, L, D), 60 + i) for i in range(4))
+    k[:, :, : L // 3] *= 3                                # popular and unpopular blocks
+    if scope != "sparse":
+        m = sla_b200.SparseLinearAttention(D, 0.1, "softmax", BLKQ, 64, linear_scope=scope).cuda()
+        with torch.no_grad():
+            m.proj_l.weight.copy_(_randn((D, D), 70, torch.float32) * 0.05)
+
+    def grads(h0, h1):
+        qs, ks, vs = (t[:, h0:h1].contiguous().requires_grad_(True) for t in (q, k, v))
+        if scope == "sparse":
+            smap, lut, topk = sla_b200.get_block_map(qs.detach(), ks.detach(), 0.1, BLKQ, 64)
+            o = sla_b200._attention.apply(qs, ks, vs, smap, lut, topk, BLKQ, 64)
+        else:
+            o = m(qs, ks, vs)
+        o.backward(do[:, h0:h1].contiguous())
+        return qs.grad, ks.grad, vs.grad
+
+    whole = grads(0, heads)
+    for h in range(heads):
+        for a, b in zip(whole, grads(h, h + 1)):
+            assert torch.equal(a[:, h], b[:, 0])
